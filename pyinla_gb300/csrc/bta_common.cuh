@@ -561,6 +561,39 @@ __device__ __forceinline__ double rcp3_fma(double d) {
   return fma(y, fma(e, e, e), y);
 }
 
+// 1/d on the integer pipe, for a chain that waits on every reciprocal: an FP64 instruction
+// takes 64 cycles, so rcp3_fma costs 227 cycles (measured, dependent), this 120 with the
+// same error (at most 1.11e-16 relative over 2^20 values).  rcp_seed starts the hardware's
+// fp32 reciprocal of the leading 24 significand bits; rcp_finish takes d's significand m
+// (2^52 <= m < 2^53) and the seed Y0 (24 bits, Y0 2^-24 ~ 2^52 / m), forms delta = m Y0 -
+// 2^76 modulo 2^64 (|delta| < 2^54) and Y = Y0 2^29 (1 - delta 2^-76 + (delta 2^-76)^2),
+// the reciprocal's significand.  A positive d outside the range where d and 1/d are normal
+// numbers gives what rcp3_fma's flushing seed leads to: 0 where 1/d is subnormal, NaN for a
+// zero, subnormal or infinite d; so does a negative d or a NaN (a failed pivot anyway).
+__device__ __forceinline__ float rcp_seed(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const float f = __uint_as_float(0x3f800000u | (__funnelshift_l(lo, hi, 3) & 0x7fffffu));
+  float y;
+  asm volatile("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+  return y;
+}
+__device__ __forceinline__ double rcp_finish(double d, float seed) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  const unsigned Y0 = (min(__float_as_uint(seed), 0x3f7fffffu) & 0x7fffffu) | 0x800000u;
+  const unsigned long long t0 = (unsigned long long)lo * Y0;
+  const int dh = (int)((unsigned)(t0 >> 32) + mh * Y0);   // delta >> 32
+  const long long c = (long long)dh * (int)Y0 + (long long)__umulhi((unsigned)t0, Y0);   // (Y0 delta) >> 32
+  const unsigned sq = (unsigned)(((long long)dh * dh) >> 20);
+  const long long q2 = (long long)(((unsigned long long)sq * Y0) >> 24);
+  const long long Y = ((long long)Y0 << 29) - ((c - q2 + (1ll << 14)) >> 15);
+  const unsigned eb = (2044u << 20) - (hi & 0x7ff00000u);
+  const long long bits = (long long)((unsigned long long)eb << 32) + Y;
+  const unsigned ex = hi >> 20;
+  const int odd = ex - 2045u < 2u ? 0 : 0x7ff80000;   // (high words of 0 and NaN)
+  return ex - 1u < 2044u ? __longlong_as_double(bits) : __hiloint2double(odd, 0);
+}
+
 // Register slots of the update warps of smem_potrf.  Slot s < 14 holds column s + 2
 // (lane = row); slot s >= 14 holds the pair of columns c0 = 16 + 2 (s - 14) and c0 + 1,
 // rows 16..31 only (lane l: row 16 + (l & 15), column c0 + (l >> 4)): a column c needs
@@ -571,125 +604,170 @@ __host__ __device__ constexpr int potrf_slot_col(int s) { return s < POTRF_FULL 
 __host__ __device__ constexpr int potrf_slot_last(int s) { return s < POTRF_FULL ? s + 2 : 17 + 2 * (s - POTRF_FULL); }
 __host__ __device__ constexpr int potrf_slot_owner(int s) { return s < POTRF_FULL ? s % 3 : (s - 12) % 3; }
 
-// Update warp W (0..2; warp W + 1) of smem_potrf.  For every pivot j it first applies
-// pivot j to column j + 2 if it owns it and hands that column to the pivot warp, then
-// applies pivot j to its slots whose columns come later: a_rc -= w_rj u_cj (w_rj =
-// u_rj / d_j from the pivot warp's ring, u_cj from S).  Slot tests are compile-time, so
-// no predicated-off FMA is issued.
+// When the update warps apply which pivot to which slot: done[j][s] pivots have been
+// applied to slot s after step j (the step that starts when pivot j is published).  A step
+// applies every pivot so far to the look-ahead slot (column j + 2), and then up to
+// POTRF_BUDGET more per warp, to the slots whose columns are needed first; the pivots that
+// wait are kept (smem_potrf's Wt holds all).  Applying each pivot to every slot at once
+// made the first dozen steps wait for the update warps (eight FP64 instructions a step, 460
+// to 680 cycles against the chain's 352) that idled in the last dozen.
+constexpr int POTRF_BUDGET = 4;
+struct PotrfSchedule {
+  int done[TS][POTRF_SLOTS];
+};
+__host__ __device__ constexpr PotrfSchedule potrf_schedule() {
+  PotrfSchedule t{};
+  for (int j = 0; j < TS - 2; ++j) {
+    for (int s = 0; s < POTRF_SLOTS; ++s) t.done[j][s] = j ? t.done[j - 1][s] : 0;
+    for (int w = 0; w < 3; ++w) {
+      int left = POTRF_BUDGET;
+      for (int s = 0; s < POTRF_SLOTS; ++s) {
+        if (potrf_slot_owner(s) != w || potrf_slot_last(s) < j + 2) continue;
+        while (t.done[j][s] <= j && (potrf_slot_col(s) <= j + 2 || left > 0)) {
+          ++t.done[j][s];
+          --left;
+        }
+      }
+    }
+  }
+  return t;
+}
+
+constexpr PotrfSchedule POTRF_SCHEDULE = potrf_schedule();
+
+// The slots from s on of step J of update warp W (see potrf_update_step).
+template <int W, int J, int s>
+__device__ __forceinline__ void potrf_update_slot(double* S, const double* Wt, int lane, double (&acc)[POTRF_SLOTS]) {
+  if constexpr (potrf_slot_owner(s) == W && potrf_slot_last(s) >= J + 2) {
+    const int prow = 16 + (lane & 15), half = lane >> 4;
+    constexpr int c = potrf_slot_col(s), from = J ? POTRF_SCHEDULE.done[J ? J - 1 : 0][s] : 0,
+                  to = POTRF_SCHEDULE.done[J][s];
+    if constexpr (to > from) {
+#pragma unroll
+      for (int p = from; p < to; ++p)
+        acc[s] = s < POTRF_FULL ? fma(-Wt[p * TS + lane], S[c * LDS + p], acc[s])
+                                : fma(-Wt[p * TS + prow], S[(c + half) * LDS + p], acc[s]);
+    }
+    if constexpr (c == J + 2 || potrf_slot_last(s) == J + 2) {
+      if (s < POTRF_FULL) S[lane * LDS + c] = acc[s];
+      else if (c + half == J + 2) S[prow * LDS + c + half] = acc[s];
+      nbar_arrive_n<64>(POTRF_BAR_C + (J & 3));
+    }
+  }
+  if constexpr (s + 1 < POTRF_SLOTS) potrf_update_slot<W, J, s + 1>(S, Wt, lane, acc);
+}
+// Step J (pivot J published) of update warp W (0..2; warp W + 1) of smem_potrf: the
+// look-ahead column J + 2 first, handed to the pivot warp, then the other slots that
+// potrf_schedule gives this step: a_rc -= w_rp u_cp for the slot's next pivots p in order
+// (w_rp = u_rp / d_p from the pivot warp, u_cp from S).  Slots and pivots are compile-time,
+// so no predicated-off FMA is issued.
+template <int W, int J>
+__device__ __forceinline__ void potrf_update_step(double* S, const double* Wt, int lane,
+                                                  double (&acc)[POTRF_SLOTS]) {
+  nbar_sync(POTRF_BAR_L + (J & 7));
+  potrf_update_slot<W, J, 0>(S, Wt, lane, acc);
+  if constexpr (J + 1 < TS - 2) potrf_update_step<W, J + 1>(S, Wt, lane, acc);
+}
 template <int W>
-__device__ __forceinline__ void potrf_update_warp(double* S, const double (*wring)[TS], int lane) {
+__device__ __forceinline__ void potrf_update_warp(double* S, const double* Wt, int lane) {
   const int prow = 16 + (lane & 15), half = lane >> 4;
   double acc[POTRF_SLOTS];
 #pragma unroll
   for (int s = 0; s < POTRF_SLOTS; ++s)
     if (potrf_slot_owner(s) == W)
       acc[s] = s < POTRF_FULL ? S[lane * LDS + potrf_slot_col(s)] : S[prow * LDS + potrf_slot_col(s) + half];
-#pragma unroll
-  for (int j = 0; j < TS - 2; ++j) {
-    nbar_sync(POTRF_BAR_L + (j & 7));
-    const double wf = wring[j & 7][lane];   // w of this lane's row (full slots)
-    const double wp = wring[j & 7][prow];   // w of the pair slots' row
-#pragma unroll
-    for (int s = 0; s < POTRF_SLOTS; ++s) {   // the look-ahead column j + 2 first
-      if (potrf_slot_owner(s) != W) continue;
-      if (s < POTRF_FULL && potrf_slot_col(s) == j + 2) {
-        acc[s] = fma(-wf, S[(j + 2) * LDS + j], acc[s]);
-        S[lane * LDS + j + 2] = acc[s];
-        nbar_arrive_n<64>(POTRF_BAR_C + (j & 3));
-      } else if (s >= POTRF_FULL && (potrf_slot_col(s) == j + 2 || potrf_slot_col(s) + 1 == j + 2)) {
-        acc[s] = fma(-wp, S[(potrf_slot_col(s) + half) * LDS + j], acc[s]);
-        if (potrf_slot_col(s) + half == j + 2) S[prow * LDS + j + 2] = acc[s];
-        nbar_arrive_n<64>(POTRF_BAR_C + (j & 3));
-      }
-    }
-#pragma unroll
-    for (int s = 0; s < POTRF_SLOTS; ++s) {
-      if (potrf_slot_owner(s) != W || potrf_slot_last(s) <= j + 2) continue;
-      if (s < POTRF_FULL) acc[s] = fma(-wf, S[potrf_slot_col(s) * LDS + j], acc[s]);
-      else if (potrf_slot_col(s) > j + 2) acc[s] = fma(-wp, S[(potrf_slot_col(s) + half) * LDS + j], acc[s]);
-    }
-  }
+  potrf_update_step<W, 0>(S, Wt, lane, acc);
 }
 
 // In-place lower Cholesky of S (TS x TS; entries past n must already be identity).
 // Returns 0, or the 1-based column of the first non-positive (or NaN) pivot (the
 // tile then holds NaNs).  The strict upper triangle is zeroed.
 // The elimination runs in the square-root-free form S = U D^-1 U^T (u_rk: column k
-// after pivots 0..k-1, d_k = u_kk), and L = U D^{-1/2} is formed at the end, all
-// columns at once.  Warp 0 does nothing but the pivot chain: for pivot k it takes
+// after pivots 0..k-1, d_k = u_kk), and L = U D^{-1/2} is formed at the end.  Warp 0 does nothing but the pivot chain: for pivot k it takes
 // column k, already updated through pivot k-2 by its owner (awaited and loaded while
 // pivot k-1's reciprocal was formed), applies pivot k-1 itself
 // (it holds w_{:,k-1} = u_{:,k-1} / d_{k-1} in registers, the multiplier u_{k,k-1} is
 // one shuffle), stores u_{:,k} to S, forms 1/d_k and w_{:,k}, and hands w_{:,k} to the
-// update warps through an eight-slot ring.  That is five FP64 instructions per pivot on
-// the chain (GB300 issues one FP64 warp instruction per ~64 cycles on a sub-partition),
-// against seven for l_rk = a_rk / sqrt(d_k) with a refined reciprocal square root.
+// update warps through Wt (TS x TS scratch, row k: w_{:,k}).  The chain is bound by
+// latency: two FP64 instructions a pivot at 64 cycles, the reciprocal on the integer pipe
+// (rcp_finish: 120 cycles against 227 in FP64), the shuffles.  Its loop is rolled
+// (unrolled, the ~60 instructions a pivot run once each, at the rate of instruction fetch:
+// ~5.5 cycles an instruction), and the next column's barrier and load sit behind the seed
+// of the reciprocal, under its latency.  In the factorization kernel a tile takes 14.2k
+// cycles, ~405 a pivot (18k before the integer reciprocal, the update schedule and the
+// scaling of the first 30 columns beside the last two pivots): a column link at b = 128 or
+// 333 19.2 us instead of 20.3.
 // Warps 1-3 apply every pivot to the later columns (potrf_update_warp), the column that
 // the pivot warp needs next first; each entry receives its updates in pivot order.
 // Barrier ids rotate over 8 (pivots) and 4 (look-ahead columns): before the pivot warp
-// publishes pivot p+8 (and overwrites ring slot p & 7), each update warp has handed it
+// publishes pivot p+8 (the barrier id of pivot p again), each update warp has handed it
 // one of columns p+2 .. p+8 (seven consecutive columns have all three owners) and so
 // consumed pivot p; the pivot warp consumes look-ahead column p before it can publish
 // the pivot that look-ahead column p+4 needs.
-static __device__ int smem_potrf(double* S) {
+// Out of line: its code is ~25 KB, once per kernel is enough.
+static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_addr) {
+  double* S = reinterpret_cast<double*>(__cvta_shared_to_generic(s_addr));
+  double* Wt = reinterpret_cast<double*>(__cvta_shared_to_generic(w_addr));
   __shared__ int s_info;
-  __shared__ double s_wring[8][TS];
-  __shared__ double s_y[TS];
   const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_info = TS + 1;
   __syncthreads();
   if (g == 0) {
-    const double u0 = S[r * LDS];       // column 0 of U is column 0 of S
-    const double a1 = S[r * LDS + 1];   // column 1 takes no update before pivot 0
-    double dk = __shfl_sync(0xffffffffu, u0, 0);   // lane k keeps d_k
-    if (r == 0 && !positive_bits(dk)) atomicMin(&s_info, 1);
-    double wp = u0 * rcp3_fma(dk);
-    s_wring[0][r] = wp;
-    nbar_arrive(POTRF_BAR_L);
-    double a = a1;
-    double ub = __shfl_sync(0xffffffffu, u0, 1);   // u_{1,0}
-#pragma unroll
-    for (int k = 1; k < TS; ++k) {
-      a = fma(-wp, ub, a);   // column k through pivot k-1
-      const double u = (r >= k) ? a : 0.0;
+    double a = S[r * LDS];         // column k through pivot k-1 (column 0 of U is column 0 of S)
+    double an = S[r * LDS + 1];    // column k+1 through pivot k-1 (column 1: no update yet)
+    double dk = 1.0;               // lane k keeps d_k
+#pragma unroll 1
+    for (int k = 0; k < TS; ++k) {
       const double d = __shfl_sync(0xffffffffu, a, k);
-      if (r == k) dk = d;
-      S[r * LDS + k] = u;
-      if (r == 0 && !positive_bits(d)) atomicMin(&s_info, k + 1);
-      if (k < TS - 1) {
-        const double sk = rcp3_fma(d);
-        // Column k+1, updated through pivot k-1 by its owner, is awaited and loaded
-        // while this pivot's reciprocal is formed, off the chain.
+      const double ub = __shfl_sync(0xffffffffu, a, (k + 1) & 31);   // u_{k+1,k}
+      const float seed = rcp_seed(d);
+      // Column k+1, updated through pivot k-1 by its owner, is awaited and loaded while
+      // this pivot's reciprocal is formed, off the chain.
+      if (k >= 1 && k < TS - 1) {
         nbar_sync_n<64>(POTRF_BAR_C + ((k - 1) & 3));
-        const double an = S[r * LDS + k + 1];
-        const double w = u * sk;
-        ub = __shfl_sync(0xffffffffu, u, k + 1);   // u_{k+1,k}
-        if (k < TS - 2) {
-          s_wring[k & 7][r] = w;
-          nbar_arrive(POTRF_BAR_L + (k & 7));
-        }
-        wp = w;
-        a = an;
+        an = S[r * LDS + k + 1];
+      }
+      const double u = r >= k ? a : 0.0;
+      S[r * LDS + k] = u;
+      if (r == k) dk = d;
+      const double w = u * rcp_finish(d, seed);
+      a = fma(-w, ub, an);
+      if (k < TS - 2) {
+        Wt[k * TS + r] = w;
+        nbar_arrive(POTRF_BAR_L + (k & 7));
       }
     }
-    s_y[r] = rsqrt3(dk);
-  } else if (g == 1) {
-    potrf_update_warp<0>(S, s_wring, r);
-  } else if (g == 2) {
-    potrf_update_warp<1>(S, s_wring, r);
-  } else {
-    potrf_update_warp<2>(S, s_wring, r);
-  }
-  __syncthreads();
+    const unsigned bad = __ballot_sync(0xffffffffu, !positive_bits(dk));
+    if (r == 0) s_info = bad ? __ffs(bad) : 0;
+    // L = U D^{-1/2}: the last two columns here, the others by warps 1-3, which have them
+    // complete two pivots earlier
+    const double y = rsqrt3(dk);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {   // L = U D^{-1/2}: warp g scales columns g + 4q
-    const int cc = g + 4 * q;
-    S[r * LDS + cc] *= s_y[cc];
+    for (int c = TS - 2; c < TS; ++c) S[r * LDS + c] *= __shfl_sync(0xffffffffu, y, c);
+  } else {
+    if (g == 1)
+      potrf_update_warp<0>(S, Wt, r);
+    else if (g == 2)
+      potrf_update_warp<1>(S, Wt, r);
+    else
+      potrf_update_warp<2>(S, Wt, r);
+    // (each warp scales its columns from the diagonal it finds there before any is scaled)
+    const double y = rsqrt3(S[r * LDS + r]);
+    nbar_sync_n<NT - 32>(POTRF_BAR_L + 2);
+#pragma unroll
+    for (int q = 0; q < (TS - 2) / 3; ++q) {
+      const int c = 3 * q + g - 1;
+      S[r * LDS + c] *= __shfl_sync(0xffffffffu, y, c);
+    }
   }
   __syncthreads();
   const int info = s_info;
   __syncthreads();
-  return info > TS ? 0 : info;
+  return info;
+}
+
+// (the call passes shared-window addresses, so that the body's accesses are shared ones)
+static __device__ __forceinline__ int smem_potrf(double* S, double* Wt) {
+  return smem_potrf_at((unsigned)__cvta_generic_to_shared(S), (unsigned)__cvta_generic_to_shared(Wt));
 }
 
 // X <- X * F^{-T} with F lower triangular; rd = 1/diag(F) (tile_diag_recip).  Row r

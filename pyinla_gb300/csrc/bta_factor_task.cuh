@@ -321,7 +321,7 @@ static __device__ __forceinline__ bool factor_fp64_task(const FactorArgs& p, int
         const int rr = idx / TS, cc = idx % TS;
         if (rr >= g.a || cc >= g.a) X[rr * LDS + cc] = (rr == cc) ? 1.0 : 0.0;
       }
-      const int info = smem_potrf(X);
+      const int info = smem_potrf(X, F);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, g.nt * g.b + info);
@@ -423,7 +423,7 @@ static __device__ __forceinline__ bool factor_fp64_task(const FactorArgs& p, int
 
     if (type == FT_DIAG) {
       tile_pad_identity(X, g.vrows(col));
-      const int info = smem_potrf(X);
+      const int info = smem_potrf(X, F);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, i * g.b + col * TS + info);
@@ -545,7 +545,7 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
         const int rr = idx / TS, cc = idx % TS;
         if (rr >= g.a || cc >= g.a) X[rr * LDS + cc] = (rr == cc) ? 1.0 : 0.0;
       }
-      const int info = smem_potrf(X);
+      const int info = smem_potrf(X, F);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, g.nt * g.b + info);
@@ -727,7 +727,7 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
 
     if (type == FT_DIAG) {
       tile_pad_identity(X, g.vrows(col));
-      const int info = smem_potrf(X);
+      const int info = smem_potrf(X, F);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, i * g.b + col * TS + info);
