@@ -60,6 +60,7 @@ struct gbta_solver {
   double* d_arrow_part = nullptr;
   int* d_faux = nullptr;      // feeder "products done" flags [nt*B]
   int* d_dpre = nullptr;      // diagonal and feeder tiles' "partial stored" flags [2*nt*B]
+  double* d_wpub = nullptr;   // pivots of the diagonal tiles as they form [nt*B][32*32]
   int* d_kf = nullptr;        // first nonzero column tile per coupling-slot row tile [(nt-1)*B]
   bool fac_digits = false;    // d_digits holds the digit planes of the current factor
   // Overlapped selected inversion (gbta_set_selinv_overlap): the inversion runs on a
@@ -339,6 +340,7 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
   CREATE_CUDA(cudaMalloc(&s->d_stasks_m, stm.size() * sizeof(int4)));
   CREATE_CUDA(cudaMalloc(&s->d_tip_part, ntile * gbta::TS * gbta::TS * sizeof(double)));
   CREATE_CUDA(cudaMalloc(&s->d_arrow_part, ntile * gbta::TS * gbta::SOLVE_NC * sizeof(double)));
+  CREATE_CUDA(cudaMalloc(&s->d_wpub, gbta::factor_wpub_bytes(s->g)));
   CREATE_CUDA(cudaMalloc(&s->d_faux, ntile * sizeof(int)));
   CREATE_CUDA(cudaMemsetAsync(s->d_faux, 0, ntile * sizeof(int), s->stream));
   CREATE_CUDA(cudaMalloc(&s->d_dpre, 2 * ntile * sizeof(int)));
@@ -354,7 +356,7 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
   CREATE_CUDA(cudaStreamSynchronize(s->stream));
 #undef CREATE_CUDA
   s->ws_bytes = 2 * (CTRL_INTS * sizeof(int) + (size_t)nflags * sizeof(int)) + (ft.size() + st.size()) * sizeof(int4) +
-                ntile * gbta::TS * (gbta::TS + gbta::SOLVE_NC) * sizeof(double) + (nt + 2) * sizeof(double) +
+                ntile * gbta::TS * (gbta::TS + gbta::SOLVE_NC) * sizeof(double) + gbta::factor_wpub_bytes(s->g) + (nt + 2) * sizeof(double) +
                 3 * ntile * sizeof(int) + (size_t)(nt - 1) * s->g.B * sizeof(int);
   *out = s;
   g_last_error.clear();
@@ -375,6 +377,7 @@ int gbta_destroy(gbta_solver* s) {
   cudaFree(s->d_faux);
   cudaFree(s->d_dpre);
   cudaFree(s->d_kf);
+  cudaFree(s->d_wpub);
   cudaFree(s->d_ld);
   cudaFree(s->d_sig);
   cudaFree(s->d_selws);
@@ -588,16 +591,16 @@ static int factor_async(gbta_solver* s, double* D, double* L, double* R, double*
     gbta::launch_transpose_lslots(s->g, L, s->stream);
     gbta::launch_coupling_kfirst(s->g, L, s->d_kf, s->stream);
   }
-  gbta::launch_clear_feeders(s->g, s->d_flags, s->stream);
+  gbta::launch_clear_feeders(s->g, s->d_flags, s->d_wpub, s->stream);
   const gbta::LaunchCtl lc = next_launch(s, s->n_ftasks);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[0], s->stream));
   s->fac_digits = s->method == GBTA_METHOD_OZAKI;
   if (s->method == GBTA_METHOD_OZAKI)
     gbta::launch_factor_oz(s->g, D, L, R, T, use_arrow, s->d_ftasks, s->n_ftasks, s->d_tip_part,
-                           (__half*)s->d_digits, s->d_erow, lc, s->d_faux, s->d_dpre, s->d_kf);
+                           (__half*)s->d_digits, s->d_erow, lc, s->d_faux, s->d_dpre, s->d_kf, s->d_wpub);
   else
     gbta::launch_factor(s->g, D, L, R, T, use_arrow, s->d_ftasks, s->n_ftasks, s->d_tip_part, lc, s->d_faux,
-                        s->d_dpre, s->d_kf);
+                        s->d_dpre, s->d_kf, s->d_wpub);
   GBTA_CUDA(cudaGetLastError());
   GBTA_CUDA(cudaEventRecord(s->ev_fac, s->stream));
   s->fac_evt = true;

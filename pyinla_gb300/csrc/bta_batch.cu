@@ -129,6 +129,7 @@ struct BatchInst {
   int method = GBTA_METHOD_OZAKI;
   size_t flags_off = 0;     // in ints, into the flag pool
   size_t faux_off = 0;      // in ints, into the feeder pool (flags [nt*B])
+  size_t wpub_off = 0;      // in doubles, into the pivot words
   int n_ftasks = 0, n_stasks = 0, n_vtasks = 0;
   // device workspace (inside the pool)
   int4* ftasks = nullptr;
@@ -166,6 +167,8 @@ struct gbta_batch {
   size_t nflags_total = 0;
   int* d_faux = nullptr;    // feeder "products done" flags of every instance
   size_t nfaux_total = 0;
+  double* d_wpub = nullptr; // pivot words of every instance's diagonal tiles
+  size_t wpub_bytes = 0;
   void* pool = nullptr;
   size_t pool_bytes = 0;
   int* h_ctrl = nullptr;   // pinned
@@ -267,6 +270,7 @@ int build_args(gbta_batch* bt) {
     f.feed_pre = bt->d_faux + q.faux_off;
     f.diag_pre = bt->d_faux + q.faux_off + (size_t)g.nt * g.B;
     f.kf = g.nt > 1 ? bt->d_faux + q.faux_off + 3 * (size_t)g.nt * g.B : nullptr;
+    f.wpub = bt->d_wpub + q.wpub_off;
     f.c = batch_ctl(bt, flags, EP_FACTOR);
     gbta::SelinvArgs& s = sa[k];
     const size_t bb = (size_t)g.b * g.b;
@@ -353,6 +357,7 @@ int run_async(gbta_batch* bt, int phases, double* logdet_out) {
   BATCH_CUDA(cudaMemsetAsync(bt->d_faux, 0, bt->nfaux_total * sizeof(int), st));
   const gbta::Ctl c = batch_ctl(bt, nullptr, 0);
   if (phases & GBTA_PHASE_FACTOR) {
+    BATCH_CUDA(cudaMemsetAsync(bt->d_wpub, 0xff, bt->wpub_bytes, st));   // WORD_EMPTY
     for (const BatchInst& q : bt->inst)
       if (q.g.nt > 1) {
         gbta::launch_transpose_lslots(q.g, q.L, st);
@@ -473,6 +478,8 @@ int gbta_batch_create(int n, const int* b, const int* nt, const int* a, const in
     q.faux_off = bt->nfaux_total;
     // feeder flags, diagonal- and feeder-partial flags, then the coupling slots' kfirst
     bt->nfaux_total += 3 * (size_t)g.nt * g.B + (size_t)(g.nt - 1) * g.B;
+    q.wpub_off = bt->wpub_bytes / sizeof(double);
+    bt->wpub_bytes += gbta::factor_wpub_bytes(g);
     flags_total += (size_t)g.nflags();
     const size_t ntile = (size_t)g.nt * g.B, bb = (size_t)g.b * g.b;
     o_ft[k] = off;
@@ -508,6 +515,7 @@ int gbta_batch_create(int n, const int* b, const int* nt, const int* a, const in
   CREATE_CUDA(cudaMalloc(&bt->pool, off));
   CREATE_CUDA(cudaMalloc(&bt->d_flags, flags_total * sizeof(int)));
   CREATE_CUDA(cudaMalloc(&bt->d_faux, bt->nfaux_total * sizeof(int)));
+  CREATE_CUDA(cudaMalloc(&bt->d_wpub, bt->wpub_bytes));
   CREATE_CUDA(cudaMalloc(&bt->d_ctrl, CTRL_INTS * sizeof(int)));
   CREATE_CUDA(cudaMalloc(&bt->d_info, n * sizeof(int)));
   CREATE_CUDA(cudaMallocHost(&bt->h_ctrl, CTRL_INTS * sizeof(int)));
@@ -558,6 +566,7 @@ int gbta_batch_destroy(gbta_batch* bt) {
   cudaFree(bt->pool);
   cudaFree(bt->d_flags);
   cudaFree(bt->d_faux);
+  cudaFree(bt->d_wpub);
   cudaFree(bt->d_ctrl);
   cudaFree(bt->d_info);
   cudaFree(bt->d_fargs);
@@ -574,7 +583,7 @@ int gbta_batch_destroy(gbta_batch* bt) {
 }
 
 size_t gbta_batch_workspace_bytes(const gbta_batch* bt) {
-  return bt ? bt->pool_bytes + (bt->nflags_total + bt->nfaux_total) * sizeof(int) : 0;
+  return bt ? bt->pool_bytes + bt->wpub_bytes + (bt->nflags_total + bt->nfaux_total) * sizeof(int) : 0;
 }
 
 int gbta_batch_set_stream(gbta_batch* bt, void* stream) {

@@ -57,6 +57,19 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
   asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
+// Words that carry their own readiness: a buffer is filled with WORD_EMPTY (a NaN with its
+// sign set, which no arithmetic instruction returns), its producer writes each word once and
+// a consumer polls the words it needs.  A hop is then one store and one load, without the
+// release, the flag and the reload of a published tile.
+constexpr long long WORD_EMPTY = -1ll;
+__device__ __forceinline__ void st_word(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ long long ld_word(const double* p) {
+  long long v;
+  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ int ld_relaxed(const int* p) {
   return *(volatile const int*)p;
 }
@@ -130,6 +143,34 @@ static __device__ bool spin_ready(const Ctl& c, const int* flag, int* seen = nul
       if (dt > SPIN_NS) __nanosleep(256);
     }
   }
+}
+
+// This thread: wait (bounded as spin_ready) for a word of a WORD_EMPTY-filled buffer.
+// (the polling loop is out of line: its callers sit in unrolled code)
+static __device__ __noinline__ long long poll_word(int* ctrl, unsigned long long wait_ns, const double* p) {
+  const Ctl c{ctrl, nullptr, 0, wait_ns, nullptr};
+  long long x = ld_word(p);
+  if (x == WORD_EMPTY) {
+    const unsigned long long t0 = gtimer();
+    for (unsigned it = 1; (x = ld_word(p)) == WORD_EMPTY; ++it) {
+      if ((it & 63) == 0) {
+        if (ld_relaxed(c.ctrl + CTRL_ABORT)) return WORD_EMPTY;
+        const unsigned long long dt = gtimer() - t0;
+        if (dt > c.wait_ns) {
+          atomicCAS(c.ctrl + CTRL_ERR, ERR_NONE, ERR_TIMEOUT);
+          raise_abort(c);
+          return WORD_EMPTY;
+        }
+        if (dt > SPIN_NS) __nanosleep(256);
+      }
+    }
+  }
+  return x;
+}
+static __device__ __forceinline__ bool wait_word(const Ctl& c, const double* p, double& v) {
+  const long long x = poll_word(c.ctrl, c.wait_ns, p);
+  v = __longlong_as_double(x);
+  return x != WORD_EMPTY;
 }
 
 // CTA-wide wait on up to two flags (nullptr = no flag).  All threads return the
@@ -704,8 +745,11 @@ __device__ __forceinline__ void potrf_update_warp(double* S, const double* Wt, i
 // one of columns p+2 .. p+8 (seven consecutive columns have all three owners) and so
 // consumed pivot p; the pivot warp consumes look-ahead column p before it can publish
 // the pivot that look-ahead column p+4 needs.
+// With Wg (TS x TS words of global memory holding WORD_EMPTY) every pivot k is also written
+// there as it forms, row k: w_{:,k} with d_k in w_kk's place, for tasks on other SMs that
+// follow the elimination (wait_word).
 // Out of line: its code is ~25 KB, once per kernel is enough.
-static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_addr) {
+static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_addr, double* Wg) {
   double* S = reinterpret_cast<double*>(__cvta_shared_to_generic(s_addr));
   double* Wt = reinterpret_cast<double*>(__cvta_shared_to_generic(w_addr));
   __shared__ int s_info;
@@ -735,6 +779,7 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
         Wt[k * TS + r] = w;
         nbar_arrive(POTRF_BAR_L + (k & 7));
       }
+      if (Wg) st_word(Wg + k * TS + r, r == k ? d : w);
     }
     const unsigned bad = __ballot_sync(0xffffffffu, !positive_bits(dk));
     if (r == 0) s_info = bad ? __ffs(bad) : 0;
@@ -766,8 +811,8 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
 }
 
 // (the call passes shared-window addresses, so that the body's accesses are shared ones)
-static __device__ __forceinline__ int smem_potrf(double* S, double* Wt) {
-  return smem_potrf_at((unsigned)__cvta_generic_to_shared(S), (unsigned)__cvta_generic_to_shared(Wt));
+static __device__ __forceinline__ int smem_potrf(double* S, double* Wt, double* Wg = nullptr) {
+  return smem_potrf_at((unsigned)__cvta_generic_to_shared(S), (unsigned)__cvta_generic_to_shared(Wt), Wg);
 }
 
 // X <- X * F^{-T} with F lower triangular; rd = 1/diag(F) (tile_diag_recip).  Row r
@@ -824,6 +869,131 @@ static __device__ void smem_trsm_rlt_rows8(double* X, const double* FS, const do
   X[row * LDS + cg] = a0;
   X[row * LDS + cg + 16] = a1;
   __syncthreads();
+}
+
+// ---- solves that follow the factorization of their diagonal tile ------------------
+// X <- X F^{-T} computed while the diagonal tile is still being factored on another SM: W
+// (global words, see smem_potrf's Wg) gives w_kj = u_kj / d_j and d_j of pivot after pivot,
+// and y_j = s_j - sum_{i<j} y_i w_ji, x_j = y_j / sqrt(d_j) is the solve in the
+// square-root-free form.  Waiting for the finished tile instead puts its scaling, store,
+// flag and reload and the whole solve (9.4 us for 32 rows) behind the last pivot, for every
+// tile of the column.  Four pivots, one word a thread, are staged at a time into Ws (TS x TS,
+// row j: w_:j) by follow_stage; the next four are requested before the four are used.
+struct FollowWords {
+  const double* W;
+  long long ahead;   // this thread's word of the next four pivots, as last read
+};
+__device__ __forceinline__ bool follow_begin(FollowWords& f, const Ctl& c, const double* W) {
+  double v;
+  bool ok = true;
+  if (threadIdx.x == 0) ok = wait_word(c, W, v);   // (one thread polls until the first pivot)
+  ok = __syncthreads_and(ok);
+  f.W = W;
+  f.ahead = ld_word(W + threadIdx.x);
+  return ok;
+}
+__device__ __forceinline__ bool follow_stage(FollowWords& f, const Ctl& c, double* Ws, int j0) {
+  double v = __longlong_as_double(f.ahead);
+  bool ok = true;
+  if (f.ahead == WORD_EMPTY) ok = wait_word(c, f.W + j0 * TS + threadIdx.x, v);
+  Ws[j0 * TS + threadIdx.x] = v;
+  ok = __syncthreads_and(ok);
+  if (j0 + 4 < TS) f.ahead = ld_word(f.W + (j0 + 4) * TS + threadIdx.x);
+  return ok;
+}
+
+// Rows row0 .. row0 + 7 of X (the split of smem_trsm_rlt_rows8).  Returns false, uniformly,
+// when a wait was given up.
+static __device__ __forceinline__ bool smem_trsm_follow_rows8_at(unsigned x_addr, int* ctrl, unsigned long long wait_ns,
+                                                              const double* W, unsigned ws_addr, int row0) {
+  double* X = reinterpret_cast<double*>(__cvta_shared_to_generic(x_addr));
+  double* Ws = reinterpret_cast<double*>(__cvta_shared_to_generic(ws_addr));
+  const Ctl c{ctrl, nullptr, 0, wait_ns, nullptr};
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = row0 + 2 * w + (lane >> 4), cg = lane & 15, base = lane & 16;
+  __syncthreads();
+  double a0 = X[row * LDS + cg], a1 = X[row * LDS + cg + 16];
+  double s0 = 0.0;
+  FollowWords f;
+  if (!follow_begin(f, c, W)) return false;
+#pragma unroll 1
+  for (int j0 = 0; j0 < TS; j0 += 4) {
+    if (!follow_stage(f, c, Ws, j0)) return false;
+    if (j0 < 16) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = j0 + q;
+        const double yj = __shfl_sync(0xffffffffu, a0, base | j);
+        const double f0 = Ws[j * TS + cg], f1 = Ws[j * TS + cg + 16];
+        if (cg > j) a0 = fma(-yj, f0, a0);
+        a1 = fma(-yj, f1, a1);
+      }
+    } else {
+      if (j0 == 16) s0 = rsqrt3(Ws[cg * TS + cg]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = j0 + q;
+        const double yj = __shfl_sync(0xffffffffu, a1, base | (j & 15));
+        const double f1 = Ws[j * TS + cg + 16];
+        if (cg + 16 > j) a1 = fma(-yj, f1, a1);
+      }
+    }
+  }
+  X[row * LDS + cg] = a0 * s0;
+  X[row * LDS + cg + 16] = a1 * rsqrt3(Ws[(cg + 16) * TS + cg + 16]);
+  __syncthreads();
+  return true;
+}
+
+// All 32 rows of X: warp w owns rows 8 w .. 8 w + 7, four lanes a row with columns (lane &
+// 3) + 4 q, so that a column goes to its row's lanes by one shuffle and only the staging has
+// barriers.  144 FP64 instructions a warp (9.2k cycles), under the factorization's 14k.
+// rs: TS doubles.
+static __device__ __noinline__ bool smem_trsm_follow_at(unsigned x_addr, int* ctrl, unsigned long long wait_ns,
+                                                        const double* W, unsigned ws_addr, unsigned rs_addr) {
+  double* X = reinterpret_cast<double*>(__cvta_shared_to_generic(x_addr));
+  double* Ws = reinterpret_cast<double*>(__cvta_shared_to_generic(ws_addr));
+  double* rs = reinterpret_cast<double*>(__cvta_shared_to_generic(rs_addr));
+  const Ctl c{ctrl, nullptr, 0, wait_ns, nullptr};
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = 8 * w + (lane >> 2), cg = lane & 3;
+  FollowWords f;
+  if (!follow_begin(f, c, W)) return false;   // (its barrier covers the caller's writes of X)
+  double y[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) y[q] = X[row * LDS + cg + 4 * q];
+#pragma unroll
+  for (int J = 0; J < 8; ++J) {
+    if (!follow_stage(f, c, Ws, 4 * J)) return false;
+#pragma unroll
+    for (int ph = 0; ph < 4; ++ph) {
+      const double* wj = Ws + (4 * J + ph) * TS + cg;
+      const double yj = __shfl_sync(0xffffffffu, y[J], (lane & 28) | ph);
+      if (ph < 3 && cg > ph) y[J] = fma(-yj, wj[4 * J], y[J]);
+#pragma unroll
+      for (int q = J + 1; q < 8; ++q) y[q] = fma(-yj, wj[4 * q], y[q]);
+    }
+  }
+  if (threadIdx.x < TS) rs[threadIdx.x] = rsqrt3(Ws[threadIdx.x * TS + threadIdx.x]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) X[row * LDS + cg + 4 * q] = y[q] * rs[cg + 4 * q];
+  __syncthreads();
+  return true;
+}
+
+// The 32-row solve is out of line, as smem_potrf_at (inlined, the factorization at b = 3072
+// takes 78.4 ms instead of 74.7); the row groups', on the column chain, is inlined (b = 333,
+// nt = 60: 5.66 ms against 5.80).
+static __device__ __forceinline__ bool smem_trsm_follow_rows8(double* X, const Ctl& c, const double* W, double* Ws,
+                                                              int row0) {
+  return smem_trsm_follow_rows8_at((unsigned)__cvta_generic_to_shared(X), c.ctrl, c.wait_ns, W,
+                                   (unsigned)__cvta_generic_to_shared(Ws), row0);
+}
+static __device__ __forceinline__ bool smem_trsm_follow(double* X, const Ctl& c, const double* W, double* Ws,
+                                                        double* rs) {
+  return smem_trsm_follow_at((unsigned)__cvta_generic_to_shared(X), c.ctrl, c.wait_ns, W,
+                             (unsigned)__cvta_generic_to_shared(Ws), (unsigned)__cvta_generic_to_shared(rs));
 }
 
 // FS <- F with row j scaled by rd[j] = 1/F_jj (the strict lower part is what the

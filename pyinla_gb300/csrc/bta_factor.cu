@@ -15,8 +15,11 @@ __global__ void __launch_bounds__(NT, 1) k_factor(FactorArgs p) {
   }
 }
 
-__global__ void k_clear_feeders(Geom g, int* flags) {
+__global__ void k_clear_feeders(Geom g, int* flags, longlong2* wpub) {
   const int n = g.nt * g.B;
+  const long long nw = (long long)n * TS * TS / 2;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nw; k += (long long)gridDim.x * blockDim.x)
+    wpub[k] = make_longlong2(WORD_EMPTY, WORD_EMPTY);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const int i = k / g.B, c = k - i * g.B;
     const int fk = g.feeder_kind(i, c);
@@ -84,16 +87,15 @@ void launch_coupling_kfirst(const Geom& g, const double* L, int* kf, cudaStream_
   count_launches(1);
 }
 
-void launch_clear_feeders(const Geom& g, int* flags, cudaStream_t stream) {
-  const int n = g.nt * g.B;
-  const int blocks = (n + 255) / 256;
-  k_clear_feeders<<<blocks < 1216 ? blocks : 1216, 256, 0, stream>>>(g, flags);
+void launch_clear_feeders(const Geom& g, int* flags, double* wpub, cudaStream_t stream) {
+  const int blocks = 2 * g.nt * g.B;   // (a tile's words: 512 16-byte stores)
+  k_clear_feeders<<<blocks < 1216 ? blocks : 1216, 256, 0, stream>>>(g, flags, reinterpret_cast<longlong2*>(wpub));
   count_launches(1);
 }
 
 void launch_factor(const Geom& g, double* D, double* L, double* R, double* T, int use_arrow, const int4* tasks,
                    int ntasks, double* tip_part, const LaunchCtl& lc, int* feed_aux, int* diag_pre,
-                   const int* kf) {
+                   const int* kf, double* wpub) {
   FactorArgs p;
   p.D = D;
   p.L = L;
@@ -111,6 +113,7 @@ void launch_factor(const Geom& g, double* D, double* L, double* R, double* T, in
   p.feed_pre = feed_aux;
   p.diag_pre = diag_pre;
   p.kf = kf;
+  p.wpub = wpub;
   p.c.ctrl = lc.ctrl;
   p.c.flags = lc.flags;
   p.c.epoch = lc.epoch;

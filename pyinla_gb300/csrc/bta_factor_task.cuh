@@ -48,6 +48,8 @@ struct FactorArgs {
   int* feed_pre;        // [nt*B] flag: the feeder of diagonal tile (i, c) has its products
   int* diag_pre;        // [2*nt*B] flags: diagonal tile (i, c), then the feeder of column
                         // (i, c), holds its partial products (split loops; see FT_PART)
+  double* wpub;         // [nt*B][TS*TS] pivots of every diagonal tile, written as they form
+                        // (smem_potrf's Wg; WORD_EMPTY at launch), or null without FT_FEEDQ
   const int* kf;        // [(nt-1)*B] first column tile of each coupling-slot row tile that
                         // can be nonzero (launch_coupling_kfirst), or null
   Ctl c;
@@ -157,10 +159,14 @@ static __device__ __forceinline__ Tile feeder_tile(const FactorArgs& p, int i, i
 
 // FT_FEEDQ task: rows FEED_ROWS q .. of the feeder of diagonal tile (i, col) <- their
 // products (left there by the FT_PRE task) times D_i(col, col)^{-T}, plus their digit
-// planes (tensor-core method).  Each group adds its share of the epoch to the
-// feeder's ready flag, which reaches the epoch when the last group has written.  X, F, FS: shared tiles; rd: TS doubles; erow_t: TS ints (digits only).
-static __device__ bool factor_feed_rows(const FactorArgs& p, int t, int i, int q, int col, double* X, double* F,
-                                        double* FS, double* rd, int* erow_t, int* s_ok, unsigned long long t_task0) {
+// planes (tensor-core method).  The solve follows the diagonal task's pivots word by word
+// (FactorArgs::wpub) instead of waiting for the finished tile: from the last pivot to the
+// feeder's publication 2.9 us against 7.1 us with the tile's flag, staging and solve after
+// each other.  Each group adds its share of the epoch to the feeder's ready flag, which
+// reaches the epoch when the last group has written.  X, Ws: shared tiles; erow_t: TS ints
+// (digits only).
+static __device__ bool factor_feed_rows(const FactorArgs& p, int t, int i, int q, int col, double* X, double* Ws,
+                                        int* erow_t, int* s_ok, unsigned long long t_task0) {
   const Geom& g = p.g;
   const Ctl& c = p.c;
   int slot;
@@ -169,37 +175,16 @@ static __device__ bool factor_feed_rows(const FactorArgs& p, int t, int i, int q
   const int gc = i * g.B + col, row0 = q * FEED_ROWS;
   trace_clear_marks(c, t);
   const bool digits = p.method == GBTA_METHOD_OZAKI && p.digits;
-  // the group's rows (their products were formed ahead of the diagonal tile) are
-  // loaded while the diagonal tile is awaited
   if (!cta_wait(c, p.feed_pre + gc, nullptr, s_ok)) return false;
   constexpr int RPT = FEED_ROWS * TS / NT;
-  double xv[RPT];
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int idx = threadIdx.x + k * NT, rr = row0 + idx / TS, cc = idx % TS;
-    xv[k] = (rr < ft.rows && cc < ft.cols) ? __ldcg(ft.p + (size_t)rr * ft.ld + cc) : 0.0;
+    X[rr * LDS + cc] = (rr < ft.rows && cc < ft.cols) ? __ldcg(ft.p + (size_t)rr * ft.ld + cc) : 0.0;
   }
   if (digits && threadIdx.x < TS) erow_t[threadIdx.x] = threadIdx.x < ft.rows ? p.erow[grow0 + threadIdx.x] : 0;
-  if (!cta_wait(c, c.flags + g.fD(i, col, col), nullptr, s_ok)) return false;
-  trace_mark(c, t, 0);   // diagonal factor tile ready
-  {
-    double fv[PER_THREAD];
-    tile_ldg(fv, btile(Dblk(p, i), g, col, col));
-    tile_sts(F, fv);
-#pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int idx = threadIdx.x + k * NT;
-      X[(row0 + idx / TS) * LDS + idx % TS] = xv[k];
-    }
-  }
-  __syncthreads();
-  tile_pad_identity(F, g.vrows(col));
-  __syncthreads();
-  tile_diag_recip(F, rd);
-  __syncthreads();
-  tile_scale_rows_by_recip(FS, F, rd);
-  trace_mark(c, t, 1);   // operands staged
-  smem_trsm_rlt_rows8(X, FS, rd, row0);
+  trace_mark(c, t, 0);   // the rows' products staged
+  if (!smem_trsm_follow_rows8(X, c, p.wpub + (size_t)gc * TS * TS, Ws, row0)) return false;
   trace_mark(c, t, 2);   // rows solved
   for (int idx = threadIdx.x; idx < FEED_ROWS * TS; idx += NT) {
     const int rr = row0 + idx / TS, cc = idx % TS;
@@ -296,7 +281,7 @@ static __device__ __forceinline__ bool factor_fp64_task(const FactorArgs& p, int
     const int dmode = (tk.x & FT_PART) ? 1 : ((tk.x & FT_TAIL) ? 2 : 0);
     int* part_flag = (type == FT_DIAG ? p.diag_pre : p.diag_pre + g.nt * g.B) + i * g.B + col;
     if (!p.use_arrow && (type == FT_ARW || type == FT_TIP)) return true;
-    if (type == FT_FEEDQ) return factor_feed_rows(p, t, i, r, col, X, F, sm + 2 * TILE_SMEM, vec, nullptr, &s_ok, t_task0);
+    if (type == FT_FEEDQ) return factor_feed_rows(p, t, i, r, col, X, F, nullptr, &s_ok, t_task0);
 
     Acc acc;
     if (type == FT_TIP) {
@@ -423,7 +408,7 @@ static __device__ __forceinline__ bool factor_fp64_task(const FactorArgs& p, int
 
     if (type == FT_DIAG) {
       tile_pad_identity(X, g.vrows(col));
-      const int info = smem_potrf(X, F);
+      const int info = smem_potrf(X, F, p.wpub ? p.wpub + (size_t)(i * g.B + col) * TS * TS : nullptr);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, i * g.b + col * TS + info);
@@ -440,8 +425,12 @@ static __device__ __forceinline__ bool factor_fp64_task(const FactorArgs& p, int
     // Off-diagonal targets: X <- X * D_i(col,col)^{-T}; a structurally zero coupling tile
     // (no products, zero input) stays zero without the solve, so without its wait.
     if (!(type == FT_LOW && col < kfirst(p, lsi, r))) {
-      if (!load_diag_factor(p, i, col, F, &s_ok)) return false;
-      offdiag_trsm(X, F, sm + 2 * TILE_SMEM, vec, type == FT_ARW, g.a);
+      if (type != FT_ARW && p.wpub) {   // follow the diagonal task's pivots
+        if (!smem_trsm_follow(X, c, p.wpub + (size_t)(i * g.B + col) * TS * TS, F, vec)) return false;
+      } else {
+        if (!load_diag_factor(p, i, col, F, &s_ok)) return false;
+        offdiag_trsm(X, F, sm + 2 * TILE_SMEM, vec, type == FT_ARW, g.a);
+      }
     }
     tile_store(const_cast<double*>(tgt.p), tgt.ld, tgt.rows, tgt.cols, X);
     if (type == FT_OFFD) {
@@ -495,6 +484,153 @@ static __device__ __forceinline__ OzFactorSmem oz_factor_smem(unsigned char* raw
   return m;
 }
 
+// The product loop of a tensor-core task: X (shared FP64, the target's tile or partial) minus
+// the products of sr's steps, in place.  Out of line, with shared-window addresses and plain
+// values: inlined, its schedule -- and the throughput of every off-diagonal task -- moved by
+// up to 7 % (b = 3072) with unrelated changes of the task around it.  Returns false,
+// uniformly, when the launch is aborted.
+static __device__ __noinline__ bool oz_products_at(unsigned raw_addr, unsigned ok_addr, unsigned ready_addr,
+                                                   unsigned pipe_addr, const __half* digits, Ctl c, Geom g,
+                                                   StepRange sr, int type, int i, int r, int col, int t) {
+  auto shared_ptr = [](unsigned a) { return __cvta_shared_to_generic(a); };
+  OzPipe* pp = reinterpret_cast<OzPipe*>(shared_ptr(pipe_addr));
+  int& s_ok = *reinterpret_cast<int*>(shared_ptr(ok_addr));
+  int& s_ready = *reinterpret_cast<int*>(shared_ptr(ready_addr));
+  const OzFactorSmem sm = oz_factor_smem(reinterpret_cast<unsigned char*>(shared_ptr(raw_addr)), &s_ok, &s_ready, pp);
+  __half* stages = sm.stages;
+  double* X = sm.X;
+  const int* erow_t = sm.erow_t;
+  const int* ecol_t = sm.ecol_t;
+  OzAcc acc;
+  int esum[2][4];
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc.v[n][j] = X[oz_row(n, j) * LDS + oz_col(n, j)];
+      esum[n][j] = erow_t[oz_row(n, j)] + ecol_t[oz_col(n, j)];
+    }
+  oz_clear_partials(acc);
+
+  // ---- product loop over the final tiles left of the target (previous block
+  //      column first, then columns k < col of this block)
+  const int nsteps = sr.n;
+  const int lsi = g.lslot(i);
+  auto slots = [&](int s, int& sa, int& sb) {
+    bool isprev;
+    int pb, k;
+    step_src(g, sr, i, s, isprev, pb, k);
+    if (isprev) {
+      const int ls = g.lslot(pb);
+      sa = (type == FT_ARW) ? g.fR(pb, k) : g.fL(ls, r, k);
+      sb = g.fL(ls, col, k);
+    } else {
+      sa = (type == FT_ARW) ? g.fR(i, k) : (type == FT_LOW) ? g.fL(lsi, r, k) : g.fD(i, r, k);
+      sb = g.fD(i, col, k);
+    }
+  };
+  bool ok = true;
+  unsigned ph = pp->phase;
+  unsigned long long t_alldeps = 0;   // (trace) when the last operand was known ready
+  // stage the operand tiles (slots a, b) of a step into stage buffer st (bulk copies)
+  auto stage = [&](int st, int a_slot, int b_slot) {
+    if (threadIdx.x == 0) {
+      __half* dst = stages + st * OZF_STAGE_HALVES;
+      constexpr unsigned tb = (unsigned)(OZ_TILE * sizeof(__half));
+      oz_bulk_expect(pp, st, 2 * tb);
+      oz_bulk_copy(pp, st, dst, digits + (size_t)a_slot * OZ_TILE, tb);
+      oz_bulk_copy(pp, st, dst + OZ_OPER, digits + (size_t)b_slot * OZ_TILE, tb);
+    }
+  };
+  if (nsteps > 0) {
+    auto flags_of = [&](int s, const int*& f0, const int*& f1) {
+      int sa, sb;
+      slots(s, sa, sb);
+      f0 = c.flags + sa;
+      f1 = (sa == sb) ? nullptr : c.flags + sb;
+    };
+    int sa, sb;
+    slots(0, sa, sb);
+    ok = cta_wait(c, c.flags + sa, sa == sb ? nullptr : c.flags + sb, &s_ok);
+    if (ok) {
+      if (threadIdx.x == 0) s_ready = 1;
+      stage(0, sa, sb);
+    }
+    for (int s = 0; s < nsteps && ok; ++s) {
+      __half* cur = stages + (s & 1) * OZF_STAGE_HALVES;
+      const int nst = (s + 1) & 1;
+      {   // stage s has landed; the barrier frees stage s-1's buffers
+        const bool late = !oz_stage_wait(pp, s & 1, ph);
+        if (__syncthreads_or(late)) {
+          if (threadIdx.x == 0) {
+            atomicCAS(c.ctrl + CTRL_ERR, ERR_NONE, ERR_TIMEOUT);
+            raise_abort(c);
+          }
+          oz_stage_wait(pp, s & 1, ph);   // one more bounded wait for the copy before leaving
+          ok = false;
+          break;
+        }
+      }
+      const bool more = s + 1 < nsteps;
+      bool issued = false;
+      int na = 0, nb = 0;
+      if (more) {
+        if (s_ready <= s + 1) {   // uniform: read after the barrier, rewritten after the next one
+          __syncthreads();   // every warp has read s_ready before warp 0 advances it
+          scan_ready(c, nsteps, flags_of, &s_ready);
+          __syncthreads();
+          if (c.trace && s_ready >= nsteps && !t_alldeps) t_alldeps = gtimer();
+        }
+        if (s_ready > s + 1) {
+          slots(s + 1, na, nb);
+          stage(nst, na, nb);
+          issued = true;
+        }
+      }
+      oz_step(acc, cur, cur + OZ_OPER);
+      if ((s + 1) % OZ_CHUNK == 0) oz_fold_sub(acc, esum);   // (the last fold follows the loop)
+      if (more && !issued) {
+        slots(s + 1, na, nb);
+        if (!(ok = cta_wait(c, c.flags + na, na == nb ? nullptr : c.flags + nb, &s_ok))) break;
+        if (threadIdx.x == 0) s_ready = s + 2;
+        if (c.trace && s + 2 >= nsteps) t_alldeps = gtimer();
+        stage(nst, na, nb);
+      }
+    }
+  }
+  if (!ok) return false;   // no copy is in flight here
+  {
+    // the steps since the last fold, folded out of the loop: the short form when there
+    // are at most OZ_SHORT of them (a diagonal tail's last fold is on the column chain)
+    const int rest = nsteps % OZ_CHUNK;
+    if (rest != 0) {
+      if (rest <= OZ_SHORT)
+        oz_fold_sub_short(acc, esum);
+      else
+        oz_fold_sub(acc, esum);
+    }
+  }
+  if (threadIdx.x == 0) pp->phase = ph;
+  count_pairs(c, (unsigned long long)nsteps * oz_pairs_from(0, 0));
+  __syncthreads();
+  trace_clear_marks(c, t);
+  trace_mark(c, t, 0);   // product loop done
+  trace_put(c, t, 3, (long long)t_alldeps);   // last operand ready
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) X[oz_row(n, j) * LDS + oz_col(n, j)] = acc.v[n][j];
+  __syncthreads();
+  return true;
+}
+static __device__ __forceinline__ bool oz_products(const OzFactorSmem& sm, const __half* digits, const Ctl& c,
+                                                   const Geom& g, const StepRange& sr, int type, int i, int r, int col,
+                                                   int t) {
+  auto addr = [](const void* q) { return (unsigned)__cvta_generic_to_shared(q); };
+  return oz_products_at(addr(sm.stages), addr(sm.s_ok), addr(sm.s_ready), addr(sm.pipe), digits, c, g, sr, type, i, r,
+                        col, t);
+}
+
 // Task t of the instance described by p.  Returns false when the launch is aborted
 // (a failed pivot or a wait that ran out).
 static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t, const OzFactorSmem& sm) {
@@ -519,7 +655,7 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
     int* part_flag = (type == FT_DIAG ? p.diag_pre : p.diag_pre + g.nt * g.B) + i * g.B + col;
     if (!p.use_arrow && (type == FT_ARW || type == FT_TIP)) return true;
     if (type == FT_FEEDQ)
-      return factor_feed_rows(p, t, i, r, col, X, F, reinterpret_cast<double*>(stages), vec, erow_t, &s_ok, t_task0);
+      return factor_feed_rows(p, t, i, r, col, X, F, erow_t, &s_ok, t_task0);
     const size_t bb = (size_t)g.b * g.b, ab = (size_t)g.a * g.b;
 
     if (type == FT_TIP) {
@@ -585,128 +721,9 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
     if (dmode == 2 && !cta_wait(c, part_flag, nullptr, &s_ok)) return false;
     tile_load(X, tgt);
     __syncthreads();
-    OzAcc acc;
-    int esum[2][4];
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc.v[n][j] = X[oz_row(n, j) * LDS + oz_col(n, j)];
-        esum[n][j] = erow_t[oz_row(n, j)] + ecol_t[oz_col(n, j)];
-      }
-    oz_clear_partials(acc);
-
-    // ---- product loop over the final tiles left of the target (previous block
-    //      column first, then columns k < col of this block)
     const StepRange sr = step_range(p, type, dmode, i, r, col);
-    const int nsteps = sr.n;
     const int lsi = g.lslot(i);
-    auto slots = [&](int s, int& sa, int& sb) {
-      bool isprev;
-      int pb, k;
-      step_src(g, sr, i, s, isprev, pb, k);
-      if (isprev) {
-        const int ls = g.lslot(pb);
-        sa = (type == FT_ARW) ? g.fR(pb, k) : g.fL(ls, r, k);
-        sb = g.fL(ls, col, k);
-      } else {
-        sa = (type == FT_ARW) ? g.fR(i, k) : (type == FT_LOW) ? g.fL(lsi, r, k) : g.fD(i, r, k);
-        sb = g.fD(i, col, k);
-      }
-    };
-    bool ok = true;
-    OzPipe* pp = sm.pipe;
-    unsigned ph = pp->phase;
-    unsigned long long t_alldeps = 0;   // (trace) when the last operand was known ready
-    // stage the operand tiles (slots a, b) of a step into stage buffer st (bulk copies)
-    auto stage = [&](int st, int a_slot, int b_slot) {
-      if (threadIdx.x == 0) {
-        __half* dst = stages + st * OZF_STAGE_HALVES;
-        constexpr unsigned tb = (unsigned)(OZ_TILE * sizeof(__half));
-        oz_bulk_expect(pp, st, 2 * tb);
-        oz_bulk_copy(pp, st, dst, p.digits + (size_t)a_slot * OZ_TILE, tb);
-        oz_bulk_copy(pp, st, dst + OZ_OPER, p.digits + (size_t)b_slot * OZ_TILE, tb);
-      }
-    };
-    if (nsteps > 0) {
-      auto flags_of = [&](int s, const int*& f0, const int*& f1) {
-        int sa, sb;
-        slots(s, sa, sb);
-        f0 = c.flags + sa;
-        f1 = (sa == sb) ? nullptr : c.flags + sb;
-      };
-      int sa, sb;
-      slots(0, sa, sb);
-      ok = cta_wait(c, c.flags + sa, sa == sb ? nullptr : c.flags + sb, &s_ok);
-      if (ok) {
-        if (threadIdx.x == 0) s_ready = 1;
-        stage(0, sa, sb);
-      }
-      for (int s = 0; s < nsteps && ok; ++s) {
-        __half* cur = stages + (s & 1) * OZF_STAGE_HALVES;
-        const int nst = (s + 1) & 1;
-        {   // stage s has landed; the barrier frees stage s-1's buffers
-          const bool late = !oz_stage_wait(pp, s & 1, ph);
-          if (__syncthreads_or(late)) {
-            if (threadIdx.x == 0) {
-              atomicCAS(c.ctrl + CTRL_ERR, ERR_NONE, ERR_TIMEOUT);
-              raise_abort(c);
-            }
-            oz_stage_wait(pp, s & 1, ph);   // one more bounded wait for the copy before leaving
-            ok = false;
-            break;
-          }
-        }
-        const bool more = s + 1 < nsteps;
-        bool issued = false;
-        int na = 0, nb = 0;
-        if (more) {
-          if (s_ready <= s + 1) {   // uniform: read after the barrier, rewritten after the next one
-            __syncthreads();   // every warp has read s_ready before warp 0 advances it
-            scan_ready(c, nsteps, flags_of, &s_ready);
-            __syncthreads();
-            if (c.trace && s_ready >= nsteps && !t_alldeps) t_alldeps = gtimer();
-          }
-          if (s_ready > s + 1) {
-            slots(s + 1, na, nb);
-            stage(nst, na, nb);
-            issued = true;
-          }
-        }
-        oz_step(acc, cur, cur + OZ_OPER);
-        if ((s + 1) % OZ_CHUNK == 0) oz_fold_sub(acc, esum);   // (the last fold follows the loop)
-        if (more && !issued) {
-          slots(s + 1, na, nb);
-          if (!(ok = cta_wait(c, c.flags + na, na == nb ? nullptr : c.flags + nb, &s_ok))) break;
-          if (threadIdx.x == 0) s_ready = s + 2;
-          if (c.trace && s + 2 >= nsteps) t_alldeps = gtimer();
-          stage(nst, na, nb);
-        }
-      }
-    }
-    if (!ok) return false;   // no copy is in flight here
-    {
-      // the steps since the last fold, folded out of the loop: the short form when there
-      // are at most OZ_SHORT of them (a diagonal tail's last fold is on the column chain)
-      const int rest = nsteps % OZ_CHUNK;
-      if (rest != 0) {
-        if (rest <= OZ_SHORT)
-          oz_fold_sub_short(acc, esum);
-        else
-          oz_fold_sub(acc, esum);
-      }
-    }
-    if (threadIdx.x == 0) pp->phase = ph;
-    count_pairs(c, (unsigned long long)nsteps * oz_pairs_from(0, 0));
-    __syncthreads();
-    trace_clear_marks(c, t);
-    trace_mark(c, t, 0);   // product loop done
-    trace_put(c, t, 3, (long long)t_alldeps);   // last operand ready
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) X[oz_row(n, j) * LDS + oz_col(n, j)] = acc.v[n][j];
-    __syncthreads();
+    if (!oz_products(sm, p.digits, c, g, sr, type, i, r, col, t)) return false;
 
     if (dmode == 1) {   // a partial: stored for its tail task
       tile_store(const_cast<double*>(tgt.p), tgt.ld, tgt.rows, tgt.cols, X);
@@ -727,7 +744,7 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
 
     if (type == FT_DIAG) {
       tile_pad_identity(X, g.vrows(col));
-      const int info = smem_potrf(X, F);
+      const int info = smem_potrf(X, F, p.wpub ? p.wpub + (size_t)(i * g.B + col) * TS * TS : nullptr);
       if (info) {
         if (threadIdx.x == 0) {
           atomicCAS(info_slot, 0, i * g.b + col * TS + info);
@@ -746,14 +763,20 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
 
     // Off-diagonal targets: X <- X * D_i(col,col)^{-T}; a structurally zero coupling tile
     // (no products, zero input) stays zero without the solve, so without its wait.
+    // D and L tiles follow the diagonal task's pivots; the arrow's few rows wait for its tile.
     if (!(type == FT_LOW && col < kfirst(p, lsi, r))) {
-      if (!cta_wait(c, c.flags + g.fD(i, col, col), nullptr, &s_ok)) return false;
-      trace_mark(c, t, 1);   // diagonal factor tile ready
-      tile_load(F, make_tile(p.D + i * bb, g.b, col * TS, col * TS, g.b, g.b));
-      __syncthreads();
-      tile_pad_identity(F, g.vrows(col));
-      __syncthreads();
-      offdiag_trsm(X, F, reinterpret_cast<double*>(stages), vec, type == FT_ARW, g.a);
+      if (type != FT_ARW) {
+        trace_mark(c, t, 1);   // solve begins
+        if (!smem_trsm_follow(X, c, p.wpub + (size_t)(i * g.B + col) * TS * TS, F, vec)) return false;
+      } else {
+        if (!cta_wait(c, c.flags + g.fD(i, col, col), nullptr, &s_ok)) return false;
+        trace_mark(c, t, 1);   // diagonal factor tile ready
+        tile_load(F, make_tile(p.D + i * bb, g.b, col * TS, col * TS, g.b, g.b));
+        __syncthreads();
+        tile_pad_identity(F, g.vrows(col));
+        __syncthreads();
+        offdiag_trsm(X, F, reinterpret_cast<double*>(stages), vec, true, g.a);
+      }
       trace_mark(c, t, 2);   // triangular solve done
     }
     tile_store(const_cast<double*>(tgt.p), tgt.ld, tgt.rows, tgt.cols, X);

@@ -183,9 +183,11 @@ void count_launches(int n);
 // FT_TAIL tasks.
 // kf: (nt - 1) * B ints from launch_coupling_kfirst (the products of structurally zero
 // coupling tiles are left out), or null (every product is formed).
+// wpub: factor_wpub_bytes of pivot words (launch_clear_feeders), or null when the task list
+// has no FT_FEEDQ tasks.
 void launch_factor(const Geom& g, double* D, double* L, double* R, double* T, int use_arrow,
                    const int4* tasks, int ntasks, double* tip_part, const LaunchCtl& lc, int* feed_aux = nullptr,
-                   int* diag_pre = nullptr, const int* kf = nullptr);
+                   int* diag_pre = nullptr, const int* kf = nullptr, double* wpub = nullptr);
 
 // Transpose, in place, the L slots below the separator (slots sep() .. nt-2): before a
 // factorization they hold the caller's Q(j+1, j), afterwards the factor needs Q(j, j+1).
@@ -200,9 +202,12 @@ void launch_transpose_lslots(const Geom& g, double* L, cudaStream_t stream);
 // (after launch_transpose_lslots).  Every product with a tile k < kf is exactly zero.
 void launch_coupling_kfirst(const Geom& g, const double* L, int* kf, cudaStream_t stream);
 
-// Zero the ready flags of the feeder tiles (Geom::feeder_kind): the FT_FEEDQ tasks of
-// a factorization add shares of the epoch to them.
-void launch_clear_feeders(const Geom& g, int* flags, cudaStream_t stream);
+// Zero the ready flags of the feeder tiles (Geom::feeder_kind), to which the FT_FEEDQ
+// tasks of a factorization add shares of the epoch, and empty the pivot words they follow
+// (wpub: factor_wpub_bytes).
+void launch_clear_feeders(const Geom& g, int* flags, double* wpub, cudaStream_t stream);
+// One TS x TS tile of words per diagonal tile.
+inline size_t factor_wpub_bytes(const Geom& g) { return (size_t)g.nt * g.B * TS * TS * sizeof(double); }
 
 constexpr int SOLVE_NC = 4;   // right-hand-side columns per solve launch
 
@@ -211,7 +216,7 @@ size_t factor_oz_digit_bytes(const Geom& g);
 void launch_factor_oz(const Geom& g, double* D, double* L, double* R, double* T, int use_arrow,
                       const int4* tasks, int ntasks, double* tip_part, __half* digits, int* erow,
                       const LaunchCtl& lc, int* feed_aux = nullptr, int* diag_pre = nullptr,
-                      const int* kf = nullptr);
+                      const int* kf = nullptr, double* wpub = nullptr);
 
 // Row exponents of the input matrix (before a tensor-core factorization).
 void launch_row_exponents(const Geom& g, const double* D, const double* T, int use_arrow, int* erow,

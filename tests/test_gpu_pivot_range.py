@@ -38,3 +38,21 @@ def test_bad_pivot_is_refused(row, value):
         algs.pobtaf(D, L, R, T)
     if not np.isinf(value):
         assert f"row {row + 1})" in str(e.value)
+
+
+@pytest.mark.parametrize("b", [20, 33, 64, 97])
+def test_factor_again_after_failure_and_with_new_values(b):
+    """The pivot words that the solves follow are emptied before every factorization: a
+    handle gives each matrix its own factor, also right after a refused one."""
+    from pyinla_gb300 import algs
+    for seed in (1, 2, 3):
+        D, L, R, T, _ = orc.make_bta_c1(seed, nt=4, b=b, a=3)
+        bad = [x.copy() for x in (D, L, R, T)]
+        bad[0][1, b // 2, b // 2] = -1.0
+        with pytest.raises(np.linalg.LinAlgError):
+            algs.pobtaf(*bad)
+        ref = [x.copy() for x in (D, L, R, T)]
+        orc.pobtaf(*ref)
+        algs.pobtaf(D, L, R, T)
+        for g, r in zip((D, L, R, T), ref):
+            assert np.abs(g - r).max() <= 1e-12 * np.abs(r).max()
