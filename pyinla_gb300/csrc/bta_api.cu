@@ -650,7 +650,7 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
     // overlapped inversion its CTAs take the rest of each SM
     if (s->ctas_per_sm == 0) lc.ctas_per_sm = 1;
     if (both) {
-      gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, 0, use_arrow, s->d_arrow_part, lc, 1);
+      gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, 0, use_arrow, s->d_arrow_part, s->d_wpub, lc, 1);
     } else {
       for (int tr = (trans == 1 ? 1 : 0); tr <= (trans == 0 ? 0 : 1); ++tr) {
         if (tr == 1 && trans == 2) {   // the second sweep of trans = 2: its own launch
@@ -658,7 +658,8 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
           lc = next_launch(s, ntasks);
           if (s->ctas_per_sm == 0) lc.ctas_per_sm = 1;
         }
-        gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, tr, use_arrow, s->d_arrow_part, lc);
+        gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, tr, use_arrow, s->d_arrow_part,
+                           s->d_wpub, lc);
       }
     }
     GBTA_CUDA(cudaGetLastError());

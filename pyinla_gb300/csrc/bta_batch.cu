@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve_batch(const SolveArgs* __restri
     const int t = cta_ticket(c, &s_t);
     if (t < 0 || t >= ntotal) break;
     const int2 o = order[t];
-    if (!solve_task(inst[o.x], o.y, raw, &s_ok)) break;
+    if (!solve_task<1>(inst[o.x], o.y, raw, &s_ok)) break;   // (one right-hand side an instance)
   }
 }
 
@@ -316,6 +316,7 @@ int build_args(gbta_batch* bt) {
       v.use_arrow = use_arrow;
       v.trans = dir;
       v.part = q.arrow_part;
+      v.words = bt->d_wpub + q.wpub_off;
       v.ntasks = q.n_vtasks;
       v.both = 0;
       v.bflag0 = 0;
@@ -379,6 +380,7 @@ int run_async(gbta_batch* bt, int phases, double* logdet_out) {
     BATCH_CUDA(cudaGetLastError());
   }
   if (phases & GBTA_PHASE_SOLVE) {
+    BATCH_CUDA(cudaMemsetAsync(bt->d_wpub, 0xff, bt->wpub_bytes, st));   // WORD_EMPTY
     for (int dir = 0; dir < 2; ++dir) {
       if (int r = reset_ticket(bt)) return r;
       gbta::k_solve_batch<<<grid_of(bt, (const void*)gbta::k_solve_batch, 0, bt->n_vorder), gbta::NT, 0, st>>>(bt->d_vargs + dir * bt->n, bt->d_vorder,

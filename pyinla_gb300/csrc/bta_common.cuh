@@ -57,13 +57,15 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
   asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
-// Words that carry their own readiness: a buffer is filled with WORD_EMPTY (a NaN with its
-// sign set, which no arithmetic instruction returns), its producer writes each word once and
-// a consumer polls the words it needs.  A hop is then one store and one load, without the
-// release, the flag and the reload of a published tile.
+// Words that carry their own readiness: a buffer is filled with WORD_EMPTY (one particular
+// NaN, replaced by another when a value has its bits), its producer writes each word once
+// and a consumer polls the words it needs.  A hop is then one store and one load, without
+// the release, the flag and the reload of a published tile.
 constexpr long long WORD_EMPTY = -1ll;
 __device__ __forceinline__ void st_word(double* p, double v) {
-  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+  const long long b = __double_as_longlong(v);
+  asm volatile("st.relaxed.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(b == WORD_EMPTY ? 0x7ff8000000000000ll : b)
+               : "memory");
 }
 __device__ __forceinline__ long long ld_word(const double* p) {
   long long v;

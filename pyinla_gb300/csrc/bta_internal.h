@@ -240,8 +240,11 @@ void launch_selinv_oz(const Geom& g, const double* D, const double* L, const dou
 // both: the forward and then the backward sweep in one launch (needs 3 nt B + 2 flags,
 // solve_both_fits); trans is then ignored.
 void launch_solve(const Geom& g, const double* D, const double* L, const double* R, const double* T,
-                  double* Bv, int ldb, int nc, int trans, int use_arrow, double* arrow_part,
+                  double* Bv, int ldb, int nc, int trans, int use_arrow, double* arrow_part, double* words,
                   const LaunchCtl& lc, int both = 0);
+// words: the solution words of one launch (emptied by launch_solve); a factorization's wpub
+// buffer is large enough for SOLVE_NC columns.
+inline size_t solve_word_bytes(const Geom& g, int nc) { return 2 * (size_t)nc * g.nt * g.B * TS * sizeof(double); }
 inline bool solve_both_fits(const Geom& g) { return 3LL * g.nt * g.B + 2 <= g.nflags(); }
 
 void launch_selinv(const Geom& g, const double* D, const double* L, const double* R, const double* T,

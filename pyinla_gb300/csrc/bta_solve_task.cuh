@@ -14,8 +14,11 @@
 //   * subtract the products of every other solution tile it depends on, then
 //     u = Linv s (backward: Linv^T s);
 // leaving only  y_g = u - M y_neighbour  (one 32 x 32 matrix-vector product spread
-// over the whole CTA) between the neighbour's publication and its own.  The forward
-// sweep also leaves the arrow contribution R_i(:,r) y(i,r) of each tile in a partial
+// over the whole CTA) between the neighbour's publication and its own.  Solution tiles go
+// from task to task as words that carry their own readiness (st_word, wait_word): the chain
+// is bound by a store and a load across the chip and ~11 FP64 instructions of 64 cycles, a
+// tile's hop takes 1.40 us at b = 333 and 1.65 at b = 768 (2.3 with a store, a released
+// flag, its poll and a reload, and the additions of absent columns).  The forward sweep also leaves the arrow contribution R_i(:,r) y(i,r) of each tile in a partial
 // buffer, after publishing the tile and under a flag of its own (off the chain), and
 // the arrow task sums the partials in a fixed order.
 #pragma once
@@ -38,28 +41,34 @@ struct SolveArgs {
   int use_arrow;
   int trans;
   double* part;     // [nt*B][TS*NC] arrow partials
+  double* words;    // [nc][2][nt*B][TS] solution words (WORD_EMPTY at launch): the forward
+                    // sweep's y, then the backward sweep's x, of every column and tile
   int ntasks;       // nt*B (+1 with the arrow); both sweeps: twice that
   int both;         // one launch for the forward sweep and then the backward sweep
   int bflag0;       // (both) offset of the backward sweep's tile and arrow flags
   Ctl c;
 };
 
-static __device__ __forceinline__ int vflag(const Geom& g, int i, int r) { return i * g.B + r; }
 // Flag of the forward sweep's arrow partial of tile gi (published after the tile).
 static __device__ __forceinline__ int pflag(const Geom& g, int gi) { return g.nt * g.B + 1 + gi; }
+// Solution words of column q of tile gi in the forward (dir = 0) or backward sweep.
+static __device__ __forceinline__ double* sol_words(const SolveArgs& p, int dir, int q, int gi) {
+  return p.words + ((size_t)(2 * q + dir) * p.g.nt * p.g.B + gi) * TS;
+}
 
 // Vectors are TS x NC, stored [row][col] in shared memory (V[row*NC + col]).
 // res[q] = sum_m M[row][m] v[m][q] for q < nc, with M[row][m] = Ms[row*LDS + m]
 // (MT = false) or Ms[m*LDS + row] (MT = true).  Thread t owns row t/4 and the
 // k-range [8*(t%4), +8); the four partial sums of a row are combined with shuffles,
-// so every thread of the row returns the full dot products.
-template <bool MT>
-static __device__ __forceinline__ void cta_gemv(const double* Ms, const double* V, int nc, double (&res)[NC]) {
+// so every thread of the row returns the full dot products.  N = 1 (nc = 1) or NC: a
+// column that is not there costs the additions of its zeros otherwise (64 cycles each).
+template <bool MT, int N>
+static __device__ __forceinline__ void cta_gemv(const double* Ms, const double* V, int nc, double (&res)[N]) {
   const int row = threadIdx.x >> 2, part = threadIdx.x & 3;
 #pragma unroll
-  for (int q = 0; q < NC; ++q) {
+  for (int q = 0; q < N; ++q) {
     double s = 0.0;
-    if (q < nc) {
+    if (N == 1 || q < nc) {
 #pragma unroll
       for (int k = 0; k < TS / 4; ++k) {
         const int m = part * (TS / 4) + k;
@@ -73,18 +82,28 @@ static __device__ __forceinline__ void cta_gemv(const double* Ms, const double* 
   }
 }
 
-// Load the solution tile starting at global row `row0` (rows valid) into V.
+// V <- the solution words of tile gi (rows valid), as they are written; a barrier.  False,
+// uniformly, when a wait was given up.
+static __device__ __forceinline__ bool vec_wait(double* V, const SolveArgs& p, int dir, int gi, int rows) {
+  const int row = threadIdx.x / NC, col = threadIdx.x % NC;
+  double v = 0.0;
+  bool ok = true;
+  if (row < rows && col < p.nc) ok = wait_word(p.c, sol_words(p, dir, col, gi) + row, v);
+  V[row * NC + col] = v;
+  return __syncthreads_and(ok);
+}
+// V <- rows row0 .. of the right-hand side buffer.
 static __device__ __forceinline__ void vec_load(double* V, const SolveArgs& p, int row0, int rows) {
   const int row = threadIdx.x / NC, col = threadIdx.x % NC;
   V[row * NC + col] = (row < rows && col < p.nc) ? __ldcg(p.B + (size_t)(row0 + row) * p.ldb + col) : 0.0;
 }
 
 // Dependency of a sweep step: the matrix tile (row-major; used as is in the forward
-// sweep, transposed in the backward sweep), the solution rows it multiplies, its flag.
+// sweep, transposed in the backward sweep) and the solution tile it multiplies (vtile < 0:
+// the arrow's rows).
 struct DepTile {
   Tile t;
-  int vrow0, vrows;
-  const int* flag;
+  int vtile, vrows;
 };
 
 // Shared memory of a solve task: the diagonal factor tile Fs, Linv = F^{-1} (Ws),
@@ -93,8 +112,9 @@ struct DepTile {
 // reciprocals of the diagonal (rd).
 constexpr size_t SOLVE_SMEM = (4 * TILE_SMEM + 2 * TS * NC + TS) * sizeof(double);
 
-// Task t of a solve instance.  `raw` is SOLVE_SMEM bytes of shared memory.  Returns
-// false when the launch is aborted.
+// Task t of a solve instance with up to N columns (1 or NC).  `raw` is SOLVE_SMEM bytes of
+// shared memory.  Returns false when the launch is aborted.
+template <int N>
 static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, unsigned char* raw, int* s_okp) {
   double* Fs = reinterpret_cast<double*>(raw);
   double* Ws = Fs + TILE_SMEM;
@@ -117,6 +137,7 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
   const int fo = (p.both && !fwd) ? p.bflag0 : 0;   // offset of this sweep's flags
   const int tt = t;                                  // the ticket (trace record)
   if (p.both && !fwd) t -= nsweep;
+  const int dir = fwd ? 0 : 1;                       // region of this sweep's solution words
   {
     const unsigned long long t_task0 = c.trace ? gtimer() : 0ull;
     // ticket -> tile in the elimination order of the blocks (Geom): forward, the tiles of
@@ -206,15 +227,16 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
       }
       Ss[threadIdx.x] = s;
       __syncthreads();
-      double res[NC];
+      double res[N];
       if (fwd)
-        cta_gemv<false>(Ws, Ss, p.nc, res);
+        cta_gemv<false, N>(Ws, Ss, p.nc, res);
       else
-        cta_gemv<true>(Ws, Ss, p.nc, res);
+        cta_gemv<true, N>(Ws, Ss, p.nc, res);
       if ((threadIdx.x & 3) == 0) {
         const int row = threadIdx.x >> 2;
-        for (int q = 0; q < p.nc; ++q)
-          if (row < g.a) p.B[(size_t)(arrow_row0 + row) * p.ldb + q] = res[q];
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+          if (q < p.nc && row < g.a) p.B[(size_t)(arrow_row0 + row) * p.ldb + q] = res[q];
       }
       cta_publish(c, c.flags + fo + ntile);
       trace_task(c, tt, 1, t_task0);
@@ -242,30 +264,26 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
       if (r > 0) {
         has_nb = true;
         nb.t = make_tile(p.D + i * bb, g.b, r * TS, (r - 1) * TS, g.b, g.b);
-        nb.vrow0 = i * g.b + (r - 1) * TS;
+        nb.vtile = gi - 1;
         nb.vrows = g.vrows(r - 1);
-        nb.flag = c.flags + fo + vflag(g, i, r - 1);
       } else if (np > 0) {
         const int p0 = g.prev(i, 0);
         has_nb = true;
         nb.t = make_tile(p.L + g.lslot(p0) * bb, g.b, 0, (g.B - 1) * TS, g.b, g.b);
-        nb.vrow0 = p0 * g.b + (g.B - 1) * TS;
+        nb.vtile = p0 * g.B + g.B - 1;
         nb.vrows = g.vrows(g.B - 1);
-        nb.flag = c.flags + fo + vflag(g, p0, g.B - 1);
       }
     } else {
       if (r < g.B - 1) {
         has_nb = true;
         nb.t = make_tile(p.D + i * bb, g.b, (r + 1) * TS, r * TS, g.b, g.b);
-        nb.vrow0 = i * g.b + (r + 1) * TS;
+        nb.vtile = gi + 1;
         nb.vrows = g.vrows(r + 1);
-        nb.flag = c.flags + fo + vflag(g, i, r + 1);
       } else if (nx >= 0) {
         has_nb = true;
         nb.t = make_tile(p.L + lsi * bb, g.b, 0, r * TS, g.b, g.b);
-        nb.vrow0 = nx * g.b;
+        nb.vtile = nx * g.B;
         nb.vrows = g.vrows(0);
-        nb.flag = c.flags + fo + vflag(g, nx, 0);
       }
     }
     if (has_nb) {
@@ -287,9 +305,12 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
       }
     }
     // ---- the other dependencies (all solved before the neighbour): s -= A_k v_k
-    if (p.both && !fwd && !cta_wait(c, c.flags + vflag(g, i, r), nullptr, &s_ok)) return false;   // the forward y
-    Ss[threadIdx.x] = (srow < rows && scol < p.nc) ? __ldcg(p.B + (size_t)(row0 + srow) * p.ldb + scol) : 0.0;
-    __syncthreads();
+    if (p.both && !fwd) {   // from the forward y
+      if (!vec_wait(Ss, p, 0, gi, rows)) return false;
+    } else {
+      Ss[threadIdx.x] = (srow < rows && scol < p.nc) ? __ldcg(p.B + (size_t)(row0 + srow) * p.ldb + scol) : 0.0;
+      __syncthreads();
+    }
     int ndep, nfirst, n0 = 0;
     if (fwd) {
       // for each neighbour block p eliminated before i: S_p(r, k) y(p, k) for k < B (S_p
@@ -310,94 +331,105 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
         if (st < nfirst) {
           const int pb = g.prev(i, st < n0 ? 0 : 1), k = st < n0 ? st : st - n0;
           d.t = make_tile(p.L + g.lslot(pb) * bb, g.b, r * TS, k * TS, g.b, g.b);
-          d.vrow0 = pb * g.b + k * TS;
+          d.vtile = pb * g.B + k;
           d.vrows = g.vrows(k);
-          d.flag = c.flags + fo + vflag(g, pb, k);
         } else {
           const int k = st - nfirst;   // k < r - 1
           d.t = make_tile(p.D + i * bb, g.b, r * TS, k * TS, g.b, g.b);
-          d.vrow0 = i * g.b + k * TS;
+          d.vtile = i * g.B + k;
           d.vrows = g.vrows(k);
-          d.flag = c.flags + fo + vflag(g, i, k);
         }
       } else {
         int s2 = st;
         if (p.use_arrow && s2 == 0) {
           d.t = make_tile(p.R + i * ab, g.b, 0, r * TS, g.a, g.b);
-          d.vrow0 = arrow_row0;
+          d.vtile = -1;
           d.vrows = g.a;
-          d.flag = c.flags + fo + ntile;
         } else {
           if (p.use_arrow) --s2;
           if (s2 < nfirst) {
             const int k = g.B - 1 - s2;   // coupling slot rows B-1 down to (r == B-1 ? 1 : 0)
             d.t = make_tile(p.L + lsi * bb, g.b, k * TS, r * TS, g.b, g.b);
-            d.vrow0 = nx * g.b + k * TS;
+            d.vtile = nx * g.B + k;
             d.vrows = g.vrows(k);
-            d.flag = c.flags + fo + vflag(g, nx, k);
           } else {
             const int k = g.B - 1 - (s2 - nfirst);   // D_i rows B-1 down to r+2
             d.t = make_tile(p.D + i * bb, g.b, k * TS, r * TS, g.b, g.b);
-            d.vrow0 = i * g.b + k * TS;
+            d.vtile = i * g.B + k;
             d.vrows = g.vrows(k);
-            d.flag = c.flags + fo + vflag(g, i, k);
           }
         }
       }
       tile_load(Ts, d.t);   // the matrix tile does not depend on other tasks
-      if (!(ok = cta_wait(c, d.flag, nullptr, &s_ok))) break;
-      vec_load(Vs, p, d.vrow0, d.vrows);
-      __syncthreads();
-      double res[NC];
+      if (d.vtile >= 0) {
+        if (!(ok = vec_wait(Vs, p, dir, d.vtile, d.vrows))) break;
+      } else {
+        if (!(ok = cta_wait(c, c.flags + fo + ntile, nullptr, &s_ok))) break;
+        vec_load(Vs, p, arrow_row0, d.vrows);
+        __syncthreads();
+      }
+      double res[N];
       if (fwd)
-        cta_gemv<false>(Ts, Vs, p.nc, res);
+        cta_gemv<false, N>(Ts, Vs, p.nc, res);
       else
-        cta_gemv<true>(Ts, Vs, p.nc, res);
-      if ((threadIdx.x & 3) == 0)
-        for (int q = 0; q < p.nc; ++q) Ss[(threadIdx.x >> 2) * NC + q] -= res[q];
+        cta_gemv<true, N>(Ts, Vs, p.nc, res);
+      if ((threadIdx.x & 3) == 0) {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+          if (N == 1 || q < p.nc) Ss[(threadIdx.x >> 2) * NC + q] -= res[q];
+      }
       __syncthreads();
     }
     if (!ok) return false;
     trace_clear_marks(c, tt);
     trace_mark(c, tt, 0);   // every dependency but the neighbour done
     // u = Linv s (forward) or Linv^T s (backward)
-    double u[NC];
+    double u[N];
     if (fwd)
-      cta_gemv<false>(Ws, Ss, p.nc, u);
+      cta_gemv<false, N>(Ws, Ss, p.nc, u);
     else
-      cta_gemv<true>(Ws, Ss, p.nc, u);
+      cta_gemv<true, N>(Ws, Ss, p.nc, u);
     // ---- the neighbour: y = u - M v_nb
     if (has_nb) {
-      if (!cta_wait(c, nb.flag, nullptr, &s_ok)) return false;
-      trace_mark(c, tt, 1);   // neighbour published
-      vec_load(Vs, p, nb.vrow0, nb.vrows);
-      __syncthreads();
-      double res[NC];
-      cta_gemv<false>(Ms, Vs, p.nc, res);
+      if (!vec_wait(Vs, p, dir, nb.vtile, nb.vrows)) return false;
+      trace_mark(c, tt, 1);   // neighbour's solution here
+      double res[N];
+      cta_gemv<false, N>(Ms, Vs, p.nc, res);
 #pragma unroll
-      for (int q = 0; q < NC; ++q) u[q] -= res[q];
+      for (int q = 0; q < N; ++q) u[q] -= res[q];
     }
+    // the next tile's wait ends with these words.  (With both sweeps in one launch the
+    // right-hand side buffer only receives the backward sweep's x.)
+    if ((threadIdx.x & 3) == 0) {
+      const int row = threadIdx.x >> 2;
+#pragma unroll
+      for (int q = 0; q < N; ++q)
+        if ((N == 1 || q < p.nc) && row < rows) st_word(sol_words(p, dir, q, gi) + row, u[q]);
+    }
+    trace_mark(c, tt, 2);   // solution tile computed and published
     __syncthreads();
     if ((threadIdx.x & 3) == 0) {
       const int row = threadIdx.x >> 2;
+#pragma unroll
       for (int q = 0; q < NC; ++q) {
-        Ss[row * NC + q] = (q < p.nc && row < rows) ? u[q] : 0.0;
-        if (q < p.nc && row < rows) p.B[(size_t)(row0 + row) * p.ldb + q] = u[q];
+        const bool in = q < N && q < p.nc && row < rows;
+        const double x = q < N ? u[q < N ? q : 0] : 0.0;
+        Ss[row * NC + q] = in ? x : 0.0;
+        if (in && !(p.both && fwd)) p.B[(size_t)(row0 + row) * p.ldb + q] = x;
       }
     }
-    trace_mark(c, tt, 2);   // solution tile computed and stored
-    cta_publish(c, c.flags + fo + vflag(g, i, r));   // the next tile's wait ends here
-    trace_mark(c, tt, 3);   // published
     if (fwd && p.use_arrow) {
       // arrow partial R_i(:, r) y(i, r) (rows >= a of the staged tile are zero), off
       // the chain, under its own flag
       tile_load(Ts, make_tile(p.R + i * ab, g.b, 0, r * TS, g.a, g.b));
       __syncthreads();
-      double res[NC];
-      cta_gemv<false>(Ts, Ss, p.nc, res);
+      double res[N];
+      cta_gemv<false, N>(Ts, Ss, p.nc, res);
       if ((threadIdx.x & 3) == 0) {
         const int row = threadIdx.x >> 2;
-        for (int q = 0; q < NC; ++q) p.part[(size_t)gi * TS * NC + row * NC + q] = (q < p.nc) ? res[q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < NC; ++q)
+          p.part[(size_t)gi * TS * NC + row * NC + q] = (q < N && q < p.nc) ? res[q < N ? q : 0] : 0.0;
       }
       cta_publish(c, c.flags + pflag(g, gi));
     }
