@@ -638,17 +638,22 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
   // both sweeps in one launch where the flag array has room for the second sweep's flags
   // (every geometry but b <= 32), else one after the other
   const bool both = trans == 2 && gbta::solve_both_fits(s->g);
+  const int sweep_ctas = s->g.B * (s->g.twisted() ? 2 : 1) >= 80 ? 2 : 1;   // (see below)
   const int ntasks = (s->g.nt * s->g.B + (use_arrow ? 1 : 0)) * (both ? 2 : 1);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[4], s->stream));
   for (int c0 = 0; c0 < nrhs; c0 += gbta::SOLVE_NC) {
     const int nc = nrhs - c0 < gbta::SOLVE_NC ? nrhs - c0 : gbta::SOLVE_NC;
     if (int r = reset_ticket(s)) return r;
     gbta::LaunchCtl lc = next_launch(s, ntasks);
-    // the sweeps run one CTA per SM unless set otherwise: their chain needs few, and
-    // more spend the SMs' issue slots and memory traffic on waiting tasks (alone at
-    // nt = 128, b = 1024: 9.7 ms against 12.4 ms with as many as fit), and next to an
-    // overlapped inversion its CTAs take the rest of each SM
-    if (s->ctas_per_sm == 0) lc.ctas_per_sm = 1;
+    // The sweeps run one CTA per SM unless set otherwise: their chain needs few, and more
+    // spend the SMs' issue slots and memory traffic on waiting tasks (both sweeps at nt = 128,
+    // b = 1024: 7.0 ms against 7.9 with two and 8.7 with three).  Two where a task's other
+    // products (two block rows of tiles) take longer than the chain needs to come round to the
+    // next of the SMs it is shared out to: from 40 tiles per block edge with two chains (b =
+    // 1280: 2.49 ms against 2.59, b = 2048: 2.32 against 2.97, b = 3072: 3.08 against 4.59; b =
+    // 1024: 2.58 against 2.31), twice that with one (b = 2560: 3.61 ms either way).  Next to
+    // an overlapped inversion they leave the same two of its CTAs' places on each SM.
+    if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas;
     if (both) {
       gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, 0, use_arrow, s->d_arrow_part, s->d_wpub, lc, 1);
     } else {
@@ -656,7 +661,7 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
         if (tr == 1 && trans == 2) {   // the second sweep of trans = 2: its own launch
           if (int r = reset_ticket(s)) return r;
           lc = next_launch(s, ntasks);
-          if (s->ctas_per_sm == 0) lc.ctas_per_sm = 1;
+          if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas;
         }
         gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, tr, use_arrow, s->d_arrow_part,
                            s->d_wpub, lc);

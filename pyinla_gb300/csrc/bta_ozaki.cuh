@@ -142,10 +142,13 @@ __device__ __forceinline__ bool oz_pairs_vanish(int za, int zb) {
 
 // Write the digit planes of the valid part of a shared FP64 tile X (rows x cols)
 // to dst ([plane][row][col] halves), row r relative to 2^Eof(r).  Each thread converts
-// pairs of adjacent columns and stores them as one 32-bit word; the rest is zero.
+// pairs of adjacent columns and stores them as one 32-bit word; the rest is zero.  The loop
+// is rolled: unrolled, its ~500 instructions run once a task, at the rate of instruction
+// fetch (selected inversion at nt = 60, b = 333 5.25 -> 4.95 ms, on the 32 x 32 x 128 model
+// 44.0 -> 42.4 ms).
 template <class EOf>
 __device__ __forceinline__ void oz_store_digits_e(__half* dst, const double* X, int rows, int cols, EOf Eof) {
-#pragma unroll
+#pragma unroll 1
   for (int q = 0; q < PER_THREAD / 2; ++q) {
     const int p = threadIdx.x + q * NT;
     const int r = p / (TS / 2), c = 2 * (p % (TS / 2));
@@ -400,6 +403,15 @@ __device__ __forceinline__ void oz_step_z(OzAcc& acc, const __half* As, const __
   }
 }
 
+// ((a * 128 + b) * 128 + c) * 128 + d for the partial sums of four neighbouring diagonals, at
+// most 8 * 64^2 * 32 * OZ_CHUNK in magnitude, so that each pair fits 32 bits: one wide
+// multiply instead of three (a fold is ~400 straight-line instructions; the factorization at
+// nt = 60, b = 333 5.67 -> 5.56 ms, at nt = 12, b = 3072 74.2 -> 73.3 ms).
+static_assert(8ll * 64 * 64 * TS * OZ_CHUNK * 129 < (1ll << 31), "a pair of diagonals fits 32 bits");
+__device__ __forceinline__ long long oz_word4(int a, int b, int c, int d) {
+  return (long long)(a * 128 + b) * 16384 + (c * 128 + d);
+}
+
 // Fold the exact partial sums into the FP64 accumulator:
 // v -= sum_D p_D 2^(Ei+Ej-12-7D) (D = 0..8).
 // `esum[n][j]` = E_i + E_j of the thread's elements.  Clears the partials.
@@ -417,8 +429,8 @@ __device__ __forceinline__ void oz_fold_sub(OzAcc& acc, const int (&esum)[2][4])
       // diagonals 0..3 and 4..8 in two exact 64-bit integers (|I| < 2^24, so the high
       // word stays below 2^46 and the low one below 2^53: both convert exactly), then
       // two conversions and one FMA; diagonal 3 has weight 2^(Ei+Ej-33)
-      const long long hi = (((long long)I[0] * 128 + I[1]) * 128 + I[2]) * 128 + I[3];
-      const long long lo = ((((long long)I[4] * 128 + I[5]) * 128 + I[6]) * 128 + I[7]) * 128 + I[8];
+      const long long hi = oz_word4(I[0], I[1], I[2], I[3]);
+      const long long lo = oz_word4(I[4], I[5], I[6], I[7]) * 128 + I[8];
       const double vv = fma((double)lo, 0x1p-35, (double)hi);
       const double sc = __longlong_as_double((long long)(1023 + esum[n][j] - 33) << 52);
       acc.v[n][j] = fma(-vv, sc, acc.v[n][j]);
@@ -450,8 +462,8 @@ __device__ __forceinline__ void oz_fold_sub_short(OzAcc& acc, const int (&esum)[
         I[d] = __float2int_rn(acc.p[d][n][j]);
         acc.p[d][n][j] = 0.f;
       }
-      const long long hi = (((long long)I[0] * 128 + I[1]) * 128 + I[2]) * 128 + I[3];
-      const long long lo = ((((long long)I[4] * 128 + I[5]) * 128 + I[6]) * 128 + I[7]) * 128 + I[8];
+      const long long hi = oz_word4(I[0], I[1], I[2], I[3]);
+      const long long lo = oz_word4(I[4], I[5], I[6], I[7]) * 128 + I[8];
       const double L = __longlong_as_double(lo + 0x4338000000000000ll);
       const double H = __longlong_as_double(hi + 0x4338000000000000ll);
       const double vv = fma(L, 0x1p-35, H - (0x1.8p52 + 0x1.8p17));
