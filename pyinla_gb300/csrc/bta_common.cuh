@@ -63,8 +63,9 @@ __device__ __forceinline__ int atom_add_acq_rel(int* p, int v) {
 // the release, the flag and the reload of a published tile.
 constexpr long long WORD_EMPTY = -1ll;
 __device__ __forceinline__ void st_word(double* p, double v) {
-  const long long b = __double_as_longlong(v);
-  asm volatile("st.relaxed.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(b == WORD_EMPTY ? 0x7ff8000000000000ll : b)
+  const int hi = __double2hiint(v);   // (all ones: a NaN)
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p),
+               "d"(__hiloint2double(hi == -1 ? 0x7ff80000 : hi, __double2loint(v)))
                : "memory");
 }
 __device__ __forceinline__ long long ld_word(const double* p) {
@@ -772,10 +773,9 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
         nbar_sync_n<64>(POTRF_BAR_C + ((k - 1) & 3));
         an = S[r * LDS + k + 1];
       }
-      const double u = r >= k ? a : 0.0;
-      S[r * LDS + k] = u;
+      S[r * LDS + k] = a;   // (rows below k only; the others are left out when L is formed)
       if (r == k) dk = d;
-      const double w = u * rcp_finish(d, seed);
+      const double w = a * rcp_finish(d, seed);
       a = fma(-w, ub, an);
       if (k < TS - 2) {
         Wt[k * TS + r] = w;
@@ -789,7 +789,10 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
     // complete two pivots earlier
     const double y = rsqrt3(dk);
 #pragma unroll
-    for (int c = TS - 2; c < TS; ++c) S[r * LDS + c] *= __shfl_sync(0xffffffffu, y, c);
+    for (int c = TS - 2; c < TS; ++c) {
+      const double l = S[r * LDS + c] * __shfl_sync(0xffffffffu, y, c);
+      S[r * LDS + c] = r >= c ? l : 0.0;
+    }
   } else {
     if (g == 1)
       potrf_update_warp<0>(S, Wt, r);
@@ -803,7 +806,8 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
 #pragma unroll
     for (int q = 0; q < (TS - 2) / 3; ++q) {
       const int c = 3 * q + g - 1;
-      S[r * LDS + c] *= __shfl_sync(0xffffffffu, y, c);
+      const double l = S[r * LDS + c] * __shfl_sync(0xffffffffu, y, c);
+      S[r * LDS + c] = r >= c ? l : 0.0;
     }
   }
   __syncthreads();

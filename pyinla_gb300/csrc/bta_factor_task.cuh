@@ -186,10 +186,14 @@ static __device__ bool factor_feed_rows(const FactorArgs& p, int t, int i, int q
   trace_mark(c, t, 0);   // the rows' products staged
   if (!smem_trsm_follow_rows8(X, c, p.wpub + (size_t)gc * TS * TS, Ws, row0)) return false;
   trace_mark(c, t, 2);   // rows solved
-  for (int idx = threadIdx.x; idx < FEED_ROWS * TS; idx += NT) {
-    const int rr = row0 + idx / TS, cc = idx % TS;
-    if (rr < ft.rows && cc < ft.cols) const_cast<double*>(ft.p)[(size_t)rr * ft.ld + cc] = X[rr * LDS + cc];
-  }
+  auto store_rows = [&]() {
+    for (int idx = threadIdx.x; idx < FEED_ROWS * TS; idx += NT) {
+      const int rr = row0 + idx / TS, cc = idx % TS;
+      if (rr < ft.rows && cc < ft.cols) const_cast<double*>(ft.p)[(size_t)rr * ft.ld + cc] = X[rr * LDS + cc];
+    }
+  };
+  // (with digit planes, all that the products read, the FP64 rows follow the publication)
+  if (!digits) store_rows();
   if (digits) {
     __half* dst = p.digits + (size_t)slot * OZ_TILE;
     oz_store_digits_rows(dst, X, row0, ft.rows, ft.cols, erow_t);
@@ -209,6 +213,7 @@ static __device__ bool factor_feed_rows(const FactorArgs& p, int t, int i, int q
     const int nq = g.feeder_quarters(i, col), share = c.epoch / nq;
     red_add_release(c.flags + slot, q < nq - 1 ? share : c.epoch - (nq - 1) * share);
   }
+  if (digits) store_rows();
   trace_task(c, t, FT_FEEDQ, t_task0);
   return true;
 }
@@ -779,10 +784,11 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
       }
       trace_mark(c, t, 2);   // triangular solve done
     }
-    tile_store(const_cast<double*>(tgt.p), tgt.ld, tgt.rows, tgt.cols, X);
+    // (the products read the digit planes only: the FP64 tile follows the publication)
     oz_store_digits(p.digits + (size_t)tgt_slot * OZ_TILE, X, tgt.rows, tgt.cols, erow_t);
-    trace_mark(c, t, 3);   // tile and digits written
+    trace_mark(c, t, 3);   // digits written
     cta_publish(c, c.flags + tgt_slot);
+    tile_store(const_cast<double*>(tgt.p), tgt.ld, tgt.rows, tgt.cols, X);
     if (type == FT_ARW) {   // tip partial after the publication, as in factor_fp64_task
       arrow_tip_partial(p, i, col, X, F);
       cta_raise(c.flags + tgt_slot, 1);
