@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_batch(const FactorArgs* __rest
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
-  oz_pipe_init(&pipe);
+  oz_pipe_init(&pipe, c);
   const OzFactorSmem sm = oz_factor_smem(raw, &s_ok, &s_ready, &pipe);
   while (true) {
     const int t = cta_ticket(c, &s_t);
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(NT, 1) k_selinv_batch(const SelinvArgs* __rest
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
-  oz_pipe_init(&pipe);
+  oz_pipe_init(&pipe, c);
   while (true) {
     const int t = cta_ticket(c, &s_t);
     if (t < 0 || t >= ntotal) break;

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_oz(FactorArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
-  oz_pipe_init(&pipe);
+  oz_pipe_init(&pipe, p.c);
   const OzFactorSmem sm = oz_factor_smem(smem_raw, &s_ok, &s_ready, &pipe);
   while (true) {
     const int t = cta_ticket(p.c, &s_t);

@@ -220,11 +220,15 @@ __device__ __forceinline__ void oz_load_async(__half* sdst, const __half* gsrc) 
 // barriers and the parity of the next completion of each (kept across tasks).
 struct OzPipe {
   unsigned long long bar[2];
+  unsigned long long wait_ns;   // the launch's wait limit and control block (Ctl), for loops
+  int* ctrl;                    // at their register limit
   unsigned phase;   // bit st: parity of the next completion of stage st
 };
 
-__device__ __forceinline__ void oz_pipe_init(OzPipe* pp) {
+__device__ __forceinline__ void oz_pipe_init(OzPipe* pp, const Ctl& c) {
   if (threadIdx.x == 0) {
+    pp->wait_ns = c.wait_ns;
+    pp->ctrl = c.ctrl;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&pp->bar[0])) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&pp->bar[1])) : "memory");
     pp->phase = 0;

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(NT, OZS_CTAS_PER_SM) k_selinv_oz(SelinvArgs p)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
-  oz_pipe_init(&pipe);
+  oz_pipe_init(&pipe, p.c);
   while (true) {
     const int t = cta_ticket(p.c, &s_t);
     if (t < 0 || t >= p.ntasks) break;

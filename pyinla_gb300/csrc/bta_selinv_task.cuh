@@ -343,30 +343,36 @@ static __device__ __forceinline__ int smem_tile_exponent7(const double* X, int r
 }
 
 // The same exponent for a tile held in the OzAcc register layout (v), valid part rows x
-// cols.  Writes red (NT / 32 words) and contains one __syncthreads(): the caller's
-// earlier reads of red must be behind a barrier, and shared-memory writes made before
-// the call are visible to every thread after it.
+// cols, or (LOWER) the lower triangle of a symmetric one.  The high words decide (one
+// reduction instruction a warp); the low words only when they are all zero.  Writes red (NT /
+// 32 words) and contains one __syncthreads(): the caller's earlier reads of red must be behind
+// a barrier, and shared-memory writes made before the call are visible to every thread after it.
+template <bool LOWER = false>
 static __device__ __forceinline__ int acc_tile_exponent7(const double (&v)[2][4], int rows, int cols,
                                                          unsigned long long* red) {
-  unsigned long long m = 0;
+  auto reduce = [&](auto word) -> unsigned {
+    unsigned m = 0;
 #pragma unroll
-  for (int n = 0; n < 2; ++n)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (oz_row(n, q) < rows && oz_col(n, q) < cols) {
-        const unsigned long long a = (unsigned long long)__double_as_longlong(v[n][q]) & 0x7fffffffffffffffull;
-        m = a > m ? a : m;
-      }
+      for (int q = 0; q < 4; ++q)
+        if (oz_row(n, q) < rows && oz_col(n, q) < cols && (!LOWER || oz_row(n, q) >= oz_col(n, q)))
+          m = max(m, word(v[n][q]));
+    m = __reduce_max_sync(0xffffffffu, m);
+    unsigned* r32 = reinterpret_cast<unsigned*>(red);
+    if ((threadIdx.x & 31) == 0) r32[threadIdx.x >> 5] = m;
+    __syncthreads();
+    unsigned r = r32[0];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
-    m = x > m ? x : m;
+    for (int w = 1; w < NT / 32; ++w) r = max(r, r32[w]);
+    return r;
+  };
+  unsigned long long r = (unsigned long long)reduce([](double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; })
+                         << 32;
+  if (!r) {   // (uniform)
+    __syncthreads();
+    r = reduce([](double x) { return (unsigned)__double2loint(x); });
   }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  unsigned long long r = red[0];
-#pragma unroll
-  for (int w = 1; w < NT / 32; ++w) r = red[w] > r ? red[w] : r;
   if (!r) return NO_EXP;
   const int e = ilogb_bits(r) + 1;   // |x| < 2^e
   return e >= 0 ? 7 * ((e + 6) / 7) : -7 * ((-e) / 7);
@@ -409,9 +415,202 @@ static_assert(3 * TILE_SMEM * sizeof(double) <= OZS_STAGE * sizeof(__half), "X, 
 // 256 cover the loops of blocks up to 4096 rows (at most 2 B steps).
 constexpr int OZS_DESC = 256;
 constexpr size_t OZS_SMEM = 2 * OZS_STAGE * sizeof(__half) + TS * sizeof(double) + TS * sizeof(int) +
-                            4 * sizeof(double) + (SCAN_RING + 2) * sizeof(int) + OZS_DESC * sizeof(int2);
+                            4 * sizeof(double) + (SCAN_RING + 2) * sizeof(int) + 2 * sizeof(void*) +
+                            OZS_DESC * sizeof(int2);
 constexpr int OZS_CTAS_PER_SM = 3;
 static_assert(OZS_CTAS_PER_SM * (OZS_SMEM + 2048) <= 228 * 1024, "three CTAs per SM");
+
+// Shared-memory views of one CTA (carved from its OZS_SMEM bytes).
+struct OzSelinvSmem {
+  __half* stages;
+  double* X;      // stage 1
+  double* F;      // stage 1
+  double* W;      // stage 0 (the tip task)
+  double* rd;
+  int* ecol_t;
+  double* red4;
+  int* ring;      // flag words of the steps found ready
+  int* s_val;     // flag word of the last blocking wait, number of live steps
+  int2* sdesc;    // step descriptors (8-byte aligned)
+  const __half** planes;   // digit planes of the right (G) and left (Sigma) tiles
+};
+static __device__ __forceinline__ OzSelinvSmem oz_selinv_smem(unsigned char* raw) {
+  OzSelinvSmem m;
+  m.stages = reinterpret_cast<__half*>(raw);
+  m.X = reinterpret_cast<double*>(raw + OZS_STAGE * sizeof(__half));
+  m.F = m.X + TILE_SMEM;
+  m.W = reinterpret_cast<double*>(raw);
+  m.rd = reinterpret_cast<double*>(raw + 2 * OZS_STAGE * sizeof(__half));
+  m.ecol_t = reinterpret_cast<int*>(m.rd + TS);
+  m.red4 = reinterpret_cast<double*>(m.ecol_t + TS);
+  m.ring = reinterpret_cast<int*>(m.red4 + 4);
+  m.s_val = m.ring + SCAN_RING;
+  m.planes = reinterpret_cast<const __half**>(m.ring + SCAN_RING + 2);
+  m.sdesc = reinterpret_cast<int2*>(m.planes + 2);
+  return m;
+}
+
+// The product loop of a selected-inversion task over the np steps of sdesc: X (shared FP64) <-
+// start (a TS x TS tile in global memory, or zero; with `resume` the X it finds) minus the sum of
+// the products.  Out of line with plain values, as the factorization's (oz_products_at), with
+// the exponents formed at the folds and the rare control words and plane pointers read from
+// shared memory: the kernel runs at its register limit (168, three CTAs an SM), and together
+// with the one-pass symmetrisation this took the inversion at nt = 60, b = 333 from 4.89 to
+// 4.53 ms and on the 32 x 32 x 128 model from 42.3 to 40.3 ms.
+// Returns false, uniformly, when the launch is aborted.
+static __device__ __noinline__ bool sig_products_at(unsigned raw_addr, unsigned ok_addr, unsigned ready_addr,
+                                                    unsigned pipe_addr, int* flags, int epoch, int np, const double* start, bool resume) {
+  auto shared_ptr = [](unsigned a) { return __cvta_shared_to_generic(a); };
+  OzPipe* pp = reinterpret_cast<OzPipe*>(shared_ptr(pipe_addr));
+  int& s_ok = *reinterpret_cast<int*>(shared_ptr(ok_addr));
+  int& s_ready = *reinterpret_cast<int*>(shared_ptr(ready_addr));
+  const OzSelinvSmem m = oz_selinv_smem(reinterpret_cast<unsigned char*>(shared_ptr(raw_addr)));
+  __half* stages = m.stages;
+  const int* ecol_t = m.ecol_t;
+  int* ring = m.ring;
+  int* s_val = m.s_val;
+  const int2* sdesc = m.sdesc;
+  // (the rarely used control words are read from shared memory where they are needed)
+  auto ctl = [&]() { return Ctl{pp->ctrl, nullptr, epoch, pp->wait_ns, nullptr}; };
+  OzAcc acc;
+  oz_clear_partials(acc);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      acc.v[n][q] = start ? __ldcg(start + oz_row(n, q) * TS + oz_col(n, q))
+                          : (resume ? m.X[oz_row(n, q) * LDS + oz_col(n, q)] : 0.0);
+  if (resume) {   // (X lies in a stage buffer)
+    fence_async_smem();
+    __syncthreads();
+  }
+  int E = NO_EXP;   // running exponent of the left operand (unset)
+  // (the elements' exponents are formed at the fold, not held across the loop: the kernel runs
+  // at its register limit)
+  auto fold = [&](int steps) {
+    int esum[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) esum[n][q] = E + ecol_t[oz_col(n, q)];
+    oz_fold_sub_steps(acc, esum, steps);
+  };
+  auto left_of = [&](int s) -> int { return sdesc[s].x; };   // slot << 1 | transposed
+  auto right_of = [&](int s) -> const __half* { return m.planes[0] + (size_t)(sdesc[s].y & 0xffffff) * OZ_TILE; };
+  auto zero_planes_of = [&](int s) -> int { return sdesc[s].y >> 24; };
+  // stage step s's operands into stage buffer st with the left tile shifted by q
+  // planes: bulk copies of its leading OZ_S - q planes and of the right tile, the
+  // q planes below the shift zeroed by the CTA
+  unsigned ph = pp->phase;
+  int qst[2] = {0, 0};   // plane shift of the left tile in each stage buffer
+  auto stage = [&](int st, int lt, int q, int s) {
+    qst[st] = q;
+    __half* dst = stages + st * OZS_STAGE;
+    const unsigned abytes = q < OZ_S ? (unsigned)((OZ_S - q) * OZ_PLANE * sizeof(__half)) : 0u;
+    if (threadIdx.x == 0) {
+      oz_bulk_expect(pp, st, abytes + (unsigned)(OZ_TILE * sizeof(__half)));
+      if (abytes) oz_bulk_copy(pp, st, dst + q * OZ_PLANE, m.planes[1] + (size_t)(lt >> 1) * OZ_TILE, abytes);
+      oz_bulk_copy(pp, st, dst + OZ_OPER, right_of(s), (unsigned)(OZ_TILE * sizeof(__half)));
+    }
+    for (int idx = threadIdx.x; idx < q * (OZ_PLANE / 8); idx += NT)
+      reinterpret_cast<uint4*>(dst)[idx] = make_uint4(0u, 0u, 0u, 0u);
+    if (q) fence_async_smem();   // a later copy into this stage may cover these planes
+  };
+  // wait for stage st; a copy that never lands aborts the launch
+  auto stage_wait = [&](int st) -> bool {
+    const bool late = !oz_stage_wait(pp, st, ph);
+    if (__syncthreads_or(late)) {
+      if (threadIdx.x == 0) {
+        atomicCAS(pp->ctrl + CTRL_ERR, ERR_NONE, ERR_TIMEOUT);
+        raise_abort(ctl());
+      }
+      oz_stage_wait(pp, st, ph);   // give the copy one more bounded wait before leaving
+      return false;
+    }
+    return true;
+  };
+
+  bool ok = true;
+  int since_fold = 0;
+  unsigned npairs = 0;   // tile-pair products issued (thread 0's count is used)
+  auto flags_of = [&](int s, const int*& f0, const int*& f1) {
+    f0 = flags + (left_of(s) >> 1);
+    f1 = nullptr;
+  };
+  if (np > 0) {
+    const int lt = left_of(0);
+    ok = cta_wait_val(ctl(), flags + (lt >> 1), &s_ok, s_val);
+    int tcur = lt & 1;
+    if (ok) {
+      if (threadIdx.x == 0) s_ready = 1;
+      E = sig_exp_decode(*s_val, epoch);
+      stage(0, lt, 0, 0);
+    }
+    for (int s = 0; s < np && ok; ++s) {
+      __half* cur = stages + (s & 1) * OZS_STAGE;
+      const int nst = (s + 1) & 1;
+      if (!(ok = stage_wait(s & 1))) break;   // contains the barrier that frees the other stage
+      const bool more = s + 1 < np;
+      bool have = false;
+      int nt_ = 0;
+      int En = NO_EXP;
+      if (more) {
+        nt_ = left_of(s + 1);
+        if (s_ready <= s + 1) {   // uniform: read after the barrier, rewritten after the next one
+          __syncthreads();   // every warp has read s_ready before warp 0 advances it
+          scan_ready(ctl(), np, flags_of, &s_ready, ring);
+          __syncthreads();
+        }
+        if (s_ready > s + 1) {
+          En = sig_exp_decode(ring[(s + 1) % SCAN_RING], epoch);
+          stage(nst, nt_, En > E ? 0 : sig_shift(E, En), s + 1);
+          have = true;
+        }
+      }
+      // the left tile was staged qcur planes down: its planes below qcur are zero
+      // (all of them from OZ_S on: nothing to add)
+      const int qcur = qst[s & 1], zcur = zero_planes_of(s);
+      npairs += oz_pairs_issued(qcur, zcur);
+      if (oz_pairs_vanish(qcur, zcur)) {
+      } else if (tcur) {
+        oz_step_z<true>(acc, cur, cur + OZ_OPER, qcur, zcur);
+      } else {
+        oz_step_z<false>(acc, cur, cur + OZ_OPER, qcur, zcur);
+      }
+      ++since_fold;
+      if (more) {
+        if (!have) {
+          if (!(ok = cta_wait_val(ctl(), flags + (nt_ >> 1), &s_ok, s_val))) break;
+          if (threadIdx.x == 0) s_ready = s + 2;
+          En = sig_exp_decode(*s_val, epoch);
+        }
+        if ((En > E && En != NO_EXP) || since_fold == OZ_CHUNK) {
+          if (E > NO_EXP) fold(since_fold);
+          since_fold = 0;
+          if (En > E && En != NO_EXP) E = En;
+        }
+        if (!have) stage(nst, nt_, sig_shift(E, En), s + 1);
+        tcur = nt_ & 1;
+      }
+    }
+  }
+  if (!ok) return false;   // no copy is in flight here
+  if (np > 0 && E > NO_EXP) fold(since_fold);
+  if (threadIdx.x == 0) pp->phase = ph;
+  count_pairs(ctl(), npairs);
+  __syncthreads();
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m.X[oz_row(n, q) * LDS + oz_col(n, q)] = acc.v[n][q];
+  __syncthreads();
+  return true;
+}
+static __device__ __forceinline__ bool sig_products(unsigned char* raw, int* s_okp, int* s_readyp, OzPipe* pp,
+                                                    const SelinvArgs& p, int np, const double* start, bool resume) {
+  auto addr = [](const void* q) { return (unsigned)__cvta_generic_to_shared(q); };
+  return sig_products_at(addr(raw), addr(s_okp), addr(s_readyp), addr(pp), p.c.flags, p.c.epoch, np, start, resume);
+}
 
 // Task t of a tensor-core selected-inversion instance.  `raw` is OZS_SMEM bytes of
 // (16-byte aligned) shared memory.  Returns false when the launch is aborted.
@@ -423,16 +622,16 @@ static_assert(OZS_CTAS_PER_SM * (OZS_SMEM + 2048) <= 228 * 1024, "three CTAs per
 // a tile that raises E first folds the exact partial sums with the old E.
 static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t, unsigned char* raw, int* s_okp,
                                                       int* s_readyp, OzPipe* pp) {
-  __half* stages = reinterpret_cast<__half*>(raw);
-  double* X = reinterpret_cast<double*>(raw + OZS_STAGE * sizeof(__half));   // stage 1
-  double* F = X + TILE_SMEM;                                                 // stage 1
-  double* W = reinterpret_cast<double*>(raw);   // stage 0 (the tip task)
-  double* rd = reinterpret_cast<double*>(raw + 2 * OZS_STAGE * sizeof(__half));
-  int* ecol_t = reinterpret_cast<int*>(rd + TS);
-  double* red4 = reinterpret_cast<double*>(ecol_t + TS);
-  int* ring = reinterpret_cast<int*>(red4 + 4);   // flag words of the steps found ready
-  int* s_val = ring + SCAN_RING;                  // flag word of the last blocking wait
-  int2* sdesc = reinterpret_cast<int2*>(ring + SCAN_RING + 2);   // step descriptors (8-byte aligned)
+  const OzSelinvSmem m = oz_selinv_smem(raw);
+  __half* stages = m.stages;
+  double* X = m.X;
+  double* F = m.F;
+  double* W = m.W;
+  double* rd = m.rd;
+  int* ecol_t = m.ecol_t;
+  double* red4 = m.red4;
+  int* s_val = m.s_val;
+  int2* sdesc = m.sdesc;
   int& s_ok = *s_okp;
   int& s_ready = *s_readyp;
   const Geom& g = p.g;
@@ -466,27 +665,13 @@ static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t
       ecol_t[threadIdx.x] = cc < g.b ? p.ecol[(size_t)i * g.b + cc] : 0;
     }
     __syncthreads();
-    // ST_OFF / ST_PART: acc.v = -(sum of the products) = Sigma(j, col) (or its partial);
-    // ST_DIAG starts from C_col = F^{-T} F^{-1} (identity-padded): acc.v = C_col - Z =
-    // Sigma(col, col), symmetrised after the loop
-    OzAcc acc;
-    oz_clear_partials(acc);
-    {
-      const double* cinv_t = p.cinv + (size_t)(i * g.B + col) * TS * TS;
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          acc.v[n][q] = type == ST_DIAG ? __ldcg(cinv_t + oz_row(n, q) * TS + oz_col(n, q)) : 0.0;
+    if (threadIdx.x == 0) {   // (a barrier follows)
+      m.planes[0] = p.fdig;
+      m.planes[1] = p.sdig;
     }
-    int E = NO_EXP;   // running exponent of the left operand (unset)
-    int esum[2][4];
-    auto set_esum = [&]() {
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) esum[n][q] = E + ecol_t[oz_col(n, q)];
-    };
+    // The product loop leaves X = Sigma(j, col) or its partial (ST_OFF / ST_PART: minus the sum
+    // of the products), or C_col - Z = Sigma(col, col), not yet symmetric (ST_DIAG, from C_col =
+    // F^{-T} F^{-1}, identity-padded).
     // step s: left tile (Sigma digits, its flag slot and orientation) and right tile
     // (G digits), as a descriptor (left slot << 1 | transposed, right slot | the right
     // tile's leading zero planes << 24)
@@ -505,162 +690,43 @@ static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t
       const int rs = fac_slot(g, i, l, col);
       return make_int2((slot << 1) | (tr ? 1 : 0), rs | ((p.fdz ? p.fdz[rs] : 0) << 24));
     };
-    for (int s = threadIdx.x; s < np && s < OZS_DESC; s += NT) sdesc[s] = compute_desc(s);
-    __syncthreads();
-    // Steps whose right tile is zero contribute nothing: drop them up front (in order,
-    // by warp 0), so their left tiles are not even waited for.
-    const int np_all = np;
-    if (p.fdz && np <= OZS_DESC) {
-      if (threadIdx.x < 32) {
-        int cnt = 0;
-        for (int base = 0; base < np; base += 32) {
-          const int s = base + threadIdx.x;
-          const int2 d = s < np ? sdesc[s] : make_int2(0, OZ_S << 24);
-          const bool live = (d.y >> 24) < OZ_S;
-          const unsigned m = __ballot_sync(0xffffffffu, live);
-          __syncwarp();
-          if (live) sdesc[cnt + __popc(m & ((1u << threadIdx.x) - 1u))] = d;
-          cnt += __popc(m);
-          __syncwarp();
-        }
-        if (threadIdx.x == 0) s_val[1] = cnt;
-      }
+    for (int base = 0;; base += OZS_DESC) {   // (one round up to 4096-row blocks)
+      int n = min(np - base, OZS_DESC);
+      for (int s = threadIdx.x; s < n; s += NT) sdesc[s] = compute_desc(base + s);
       __syncthreads();
-      np = s_val[1];
-    }
-    auto desc_of = [&](int s) -> int2 { return np_all <= OZS_DESC ? sdesc[s] : compute_desc(s); };
-    auto left_of = [&](int s) -> SigTile {
-      const int2 d = desc_of(s);
-      SigTile st_;
-      st_.flag = c.flags + (d.x >> 1);
-      st_.trans = (d.x & 1) != 0;
-      return st_;
-    };
-    auto right_of = [&](int s) -> const __half* { return p.fdig + (size_t)(desc_of(s).y & 0xffffff) * OZ_TILE; };
-    auto zero_planes_of = [&](int s) -> int { return desc_of(s).y >> 24; };
-    // stage step s's operands into stage buffer st with the left tile shifted by q
-    // planes: bulk copies of its leading OZ_S - q planes and of the right tile, the
-    // q planes below the shift zeroed by the CTA
-    unsigned ph = pp->phase;
-    int qst[2] = {0, 0};   // plane shift of the left tile in each stage buffer
-    int zst[2] = {0, 0};   // leading zero planes of the right tile in each stage buffer
-    auto stage = [&](int st, const SigTile& lt, int q, int s) {
-      qst[st] = q;
-      zst[st] = zero_planes_of(s);
-      __half* dst = stages + st * OZS_STAGE;
-      const int slot = (int)(lt.flag - c.flags);
-      const unsigned abytes = q < OZ_S ? (unsigned)((OZ_S - q) * OZ_PLANE * sizeof(__half)) : 0u;
-      if (threadIdx.x == 0) {
-        oz_bulk_expect(pp, st, abytes + (unsigned)(OZ_TILE * sizeof(__half)));
-        if (abytes) oz_bulk_copy(pp, st, dst + q * OZ_PLANE, p.sdig + (size_t)slot * OZ_TILE, abytes);
-        oz_bulk_copy(pp, st, dst + OZ_OPER, right_of(s), (unsigned)(OZ_TILE * sizeof(__half)));
-      }
-      for (int idx = threadIdx.x; idx < q * (OZ_PLANE / 8); idx += NT)
-        reinterpret_cast<uint4*>(dst)[idx] = make_uint4(0u, 0u, 0u, 0u);
-      if (q) fence_async_smem();   // a later copy into this stage may cover these planes
-    };
-    // wait for stage st; a copy that never lands aborts the launch
-    auto stage_wait = [&](int st) -> bool {
-      const bool late = !oz_stage_wait(pp, st, ph);
-      if (__syncthreads_or(late)) {
-        if (threadIdx.x == 0) {
-          atomicCAS(c.ctrl + CTRL_ERR, ERR_NONE, ERR_TIMEOUT);
-          raise_abort(c);
+      // Steps whose right tile is zero contribute nothing: drop them up front (in order,
+      // by warp 0), so their left tiles are not even waited for.
+      if (p.fdz) {
+        if (threadIdx.x < 32) {
+          int cnt = 0;
+          for (int k = 0; k < n; k += 32) {
+            const int s = k + threadIdx.x;
+            const int2 d = s < n ? sdesc[s] : make_int2(0, OZ_S << 24);
+            const bool live = (d.y >> 24) < OZ_S;
+            const unsigned m = __ballot_sync(0xffffffffu, live);
+            __syncwarp();
+            if (live) sdesc[cnt + __popc(m & ((1u << threadIdx.x) - 1u))] = d;
+            cnt += __popc(m);
+            __syncwarp();
+          }
+          if (threadIdx.x == 0) s_val[1] = cnt;
         }
-        oz_stage_wait(pp, st, ph);   // give the copy one more bounded wait before leaving
-        return false;
+        __syncthreads();
+        n = s_val[1];
       }
-      return true;
-    };
-
-    bool ok = true;
-    int since_fold = 0;
-    unsigned long long npairs = 0;   // tile-pair products issued (thread 0's count is used)
-    // trace marks: m0 first operand ready, m1 end of the last blocking wait in the
-    // product loop, m2 ns spent in those waits, m3 product steps (a diagonal task
-    // overwrites m2 and m3 with the times its product loop ended and it published the
-    // next column's sub-diagonal tile)
-    unsigned long long waited = 0;
+      const double* start =
+          type == ST_DIAG && base == 0 ? p.cinv + (size_t)(i * g.B + col) * TS * TS : nullptr;
+      if (!sig_products(raw, s_okp, s_readyp, pp, p, n, start, base > 0)) return false;
+      if (base + OZS_DESC >= np) break;
+    }
     trace_clear_marks(c, t);
-    auto flags_of = [&](int s, const int*& f0, const int*& f1) {
-      f0 = left_of(s).flag;
-      f1 = nullptr;
-    };
-    if (np > 0) {
-      SigTile lt = left_of(0);
-      ok = cta_wait_val(c, lt.flag, &s_ok, s_val);
-      trace_mark(c, t, 0);
-      bool tcur = lt.trans;
-      if (ok) {
-        if (threadIdx.x == 0) s_ready = 1;
-        E = sig_exp_decode(*s_val, c.epoch);
-        set_esum();
-        stage(0, lt, 0, 0);
-      }
-      for (int s = 0; s < np && ok; ++s) {
-        __half* cur = stages + (s & 1) * OZS_STAGE;
-        const int nst = (s + 1) & 1;
-        if (!(ok = stage_wait(s & 1))) break;   // contains the barrier that frees the other stage
-        const bool more = s + 1 < np;
-        bool have = false;
-        SigTile nt_;
-        int En = NO_EXP;
-        if (more) {
-          nt_ = left_of(s + 1);
-          if (s_ready <= s + 1) {   // uniform: read after the barrier, rewritten after the next one
-            __syncthreads();   // every warp has read s_ready before warp 0 advances it
-            scan_ready(c, np, flags_of, &s_ready, ring);
-            __syncthreads();
-          }
-          if (s_ready > s + 1) {
-            En = sig_exp_decode(ring[(s + 1) % SCAN_RING], c.epoch);
-            stage(nst, nt_, En > E ? 0 : sig_shift(E, En), s + 1);
-            have = true;
-          }
-        }
-        // the left tile was staged qcur planes down: its planes below qcur are zero
-        // (all of them from OZ_S on: nothing to add)
-        const int qcur = qst[s & 1], zcur = zst[s & 1];
-        npairs += oz_pairs_issued(qcur, zcur);
-        if (oz_pairs_vanish(qcur, zcur)) {
-        } else if (tcur) {
-          oz_step_z<true>(acc, cur, cur + OZ_OPER, qcur, zcur);
-        } else {
-          oz_step_z<false>(acc, cur, cur + OZ_OPER, qcur, zcur);
-        }
-        ++since_fold;
-        if (more) {
-          if (!have) {
-            const unsigned long long w0 = c.trace ? gtimer() : 0ull;
-            if (!(ok = cta_wait_val(c, nt_.flag, &s_ok, s_val))) break;
-            if (c.trace) {
-              waited += gtimer() - w0;
-              trace_mark(c, t, 1);
-            }
-            if (threadIdx.x == 0) s_ready = s + 2;
-            En = sig_exp_decode(*s_val, c.epoch);
-          }
-          if ((En > E && En != NO_EXP) || since_fold == OZ_CHUNK) {
-            if (E > NO_EXP) oz_fold_sub_steps(acc, esum, since_fold);
-            since_fold = 0;
-            if (En > E && En != NO_EXP) {
-              E = En;
-              set_esum();
-            }
-          }
-          if (!have) stage(nst, nt_, sig_shift(E, En), s + 1);
-          tcur = nt_.trans;
-        }
-      }
-    }
-    if (!ok) return false;   // no copy is in flight here
-    if (np > 0 && E > NO_EXP) oz_fold_sub_steps(acc, esum, since_fold);   // acc.v = -(sum)
-    if (threadIdx.x == 0) pp->phase = ph;
-    count_pairs(c, npairs);
-    trace_put(c, t, 2, (long long)waited);
-    trace_put(c, t, 3, np);
-    __syncthreads();
+    trace_put(c, t, 3, np);   // product steps (a diagonal task overwrites it below)
     unsigned long long* red = reinterpret_cast<unsigned long long*>(red4);
+    double sv[2][4];   // this thread's elements of X
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sv[n][q] = X[oz_row(n, q) * LDS + oz_col(n, q)];
     auto acc_to_x = [&](double* Y, const double (&v)[2][4]) {
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -672,15 +738,12 @@ static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t
     // FP64 tile stored after (for the caller).
     if (type == ST_OFF) {
       const SigTile d = sig_dest(p, i, j, col);
-      acc_to_x(X, acc.v);
-      const int E = acc_tile_exponent7(acc.v, d.t.rows, d.t.cols, red);   // (its barrier covers X)
+      const int E = acc_tile_exponent7(sv, d.t.rows, d.t.cols, red);
       oz_store_digits_uniform(p.sdig + (size_t)(d.flag - c.flags) * OZ_TILE, X, d.t.rows, d.t.cols,
                               E == NO_EXP ? 0 : E);
       cta_publish_val(c, const_cast<int*>(d.flag), sig_exp_code(E));
       tile_store(const_cast<double*>(d.t.p), d.t.ld, d.t.rows, d.t.cols, X);
     } else if (type == ST_PART) {   // the partial sum, for the diagonal task that finishes the tile
-      acc_to_x(X, acc.v);
-      __syncthreads();
       tile_store(p.part + (size_t)(i * g.B + col) * TS * TS, TS, TS, TS, X);
       cta_publish(c, p.part_flag + i * g.B + col);
     } else {
@@ -717,20 +780,16 @@ static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t
         }
         cp_async_commit();
       }
-      // symmetrise: the lower triangle mirrored into the upper one, through X (selects
-      // only: no FP64 instruction on the chain)
-      acc_to_x(X, acc.v);
-      __syncthreads();
+      // symmetrise: the lower triangle copied into the upper one (no FP64 instruction on the
+      // chain)
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int r = oz_row(n, q), cc = oz_col(n, q);
-          if (r < cc) acc.v[n][q] = X[cc * LDS + r];
+          if (r > cc) X[cc * LDS + r] = sv[n][q];
         }
-      __syncthreads();
-      acc_to_x(X, acc.v);
-      const int Ed = acc_tile_exponent7(acc.v, d.t.rows, d.t.cols, red);   // (its barrier covers X)
+      const int Ed = acc_tile_exponent7<true>(sv, d.t.rows, d.t.cols, red);   // (its barrier covers X)
       // Merged task list: this task also finishes the sub-diagonal tile of the next
       // column, Sigma(j2, c2) of block column i2, whose last product needs this tile:
       // Sigma(j2, c2) = partial - Sigma(col, col) G(j2, c2) (the tile is symmetric, so
