@@ -291,15 +291,17 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
       // neighbour's solution element m.
       tile_load(Ts, nb.t);
       __syncthreads();
+      // (a warp takes one row at a time: the zeros of the triangular inverse are left out, half
+      // of 16k cycles of FP64 instructions)
       for (int idx = threadIdx.x; idx < TS * TS; idx += NT) {
         const int rr = idx / TS, cc = idx % TS;
         double sacc = 0.0;
         if (fwd) {
-#pragma unroll 8
-          for (int m = 0; m < TS; ++m) sacc = fma(Ws[rr * LDS + m], Ts[m * LDS + cc], sacc);
+#pragma unroll 4
+          for (int m = 0; m <= rr; ++m) sacc = fma(Ws[rr * LDS + m], Ts[m * LDS + cc], sacc);
         } else {
-#pragma unroll 8
-          for (int m = 0; m < TS; ++m) sacc = fma(Ws[m * LDS + rr], Ts[cc * LDS + m], sacc);
+#pragma unroll 4
+          for (int m = rr; m < TS; ++m) sacc = fma(Ws[m * LDS + rr], Ts[cc * LDS + m], sacc);
         }
         Ms[rr * LDS + cc] = sacc;
       }
