@@ -329,11 +329,10 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
   s->n_ftasks = (int)ft.size();
   s->n_stasks = (int)st.size();
   const size_t ntile = (size_t)nt * s->g.B;
-  CREATE_CUDA(cudaMalloc(&s->d_ctrl, CTRL_INTS * sizeof(int)));
+  CREATE_CUDA(cudaMalloc(&s->d_ctrl, 2 * CTRL_INTS * sizeof(int)));   // (both blocks: read by one copy)
+  s->d_ctrl2 = s->d_ctrl + CTRL_INTS;
   CREATE_CUDA(cudaMalloc(&s->d_flags, (size_t)nflags * sizeof(int)));
-  CREATE_CUDA(cudaMalloc(&s->d_ctrl2, CTRL_INTS * sizeof(int)));
   CREATE_CUDA(cudaMalloc(&s->d_flags2, (size_t)nflags * sizeof(int)));
-  CREATE_CUDA(cudaMemsetAsync(s->d_ctrl2, 0, CTRL_INTS * sizeof(int), s->stream));
   CREATE_CUDA(cudaMemsetAsync(s->d_flags2, 0, (size_t)nflags * sizeof(int), s->stream));
   CREATE_CUDA(cudaMalloc(&s->d_ftasks, ft.size() * sizeof(int4)));
   CREATE_CUDA(cudaMalloc(&s->d_stasks, st.size() * sizeof(int4)));
@@ -347,8 +346,8 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
   CREATE_CUDA(cudaMemsetAsync(s->d_dpre, 0, 2 * ntile * sizeof(int), s->stream));
   if (nt > 1) CREATE_CUDA(cudaMalloc(&s->d_kf, (size_t)(nt - 1) * s->g.B * sizeof(int)));
   CREATE_CUDA(cudaMalloc(&s->d_ld, (nt + 2) * sizeof(double)));
-  CREATE_CUDA(cudaMallocHost(&s->h_ctrl, CTRL_INTS * sizeof(int)));
-  CREATE_CUDA(cudaMemsetAsync(s->d_ctrl, 0, CTRL_INTS * sizeof(int), s->stream));
+  CREATE_CUDA(cudaMallocHost(&s->h_ctrl, 2 * CTRL_INTS * sizeof(int)));
+  CREATE_CUDA(cudaMemsetAsync(s->d_ctrl, 0, 2 * CTRL_INTS * sizeof(int), s->stream));
   CREATE_CUDA(cudaMemsetAsync(s->d_flags, 0, (size_t)nflags * sizeof(int), s->stream));
   CREATE_CUDA(cudaMemcpyAsync(s->d_ftasks, ft.data(), ft.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
   CREATE_CUDA(cudaMemcpyAsync(s->d_stasks, st.data(), st.size() * sizeof(int4), cudaMemcpyHostToDevice, s->stream));
@@ -390,7 +389,6 @@ int gbta_destroy(gbta_solver* s) {
   if (s->h_pairs) cudaFreeHost(s->h_pairs);
   for (cudaEvent_t ev : s->tev)
     if (ev) cudaEventDestroy(ev);
-  cudaFree(s->d_ctrl2);
   cudaFree(s->d_flags2);
   if (s->ev_fac) cudaEventDestroy(s->ev_fac);
   if (s->ev_sel) cudaEventDestroy(s->ev_sel);
@@ -542,19 +540,19 @@ size_t gbta_workspace_bytes(const gbta_solver* s) {
 
 int gbta_status(gbta_solver* s) {
   if (int r = check_solver(s)) return r;
-  GBTA_CUDA(cudaStreamSynchronize(s->stream));
+  // the sticky words of both control blocks (the side stream's: an overlapped inversion), by one
+  // copy behind the stream's work (two blocking copies after it took 22 us a call, this 12)
   GBTA_CUDA(cudaStreamSynchronize(s->side));
+  GBTA_CUDA(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, 2 * CTRL_INTS * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  GBTA_CUDA(cudaStreamSynchronize(s->stream));
   GBTA_CUDA(cudaGetLastError());
-  // the sticky words of both control blocks (the side stream's: an overlapped inversion)
   int info = 0, err = 0;
-  for (int* ctrl : {s->d_ctrl, s->d_ctrl2}) {
-    GBTA_CUDA(cudaMemcpy(s->h_ctrl, ctrl, CTRL_INTS * sizeof(int), cudaMemcpyDeviceToHost));
-    if (s->h_ctrl[CTRL_ERR] != 0) err = s->h_ctrl[CTRL_ERR];
-    if (s->h_ctrl[CTRL_INFO] != 0 && info == 0) info = s->h_ctrl[CTRL_INFO];
+  for (const int* w : {s->h_ctrl, s->h_ctrl + CTRL_INTS}) {
+    if (w[CTRL_ERR] != 0) err = w[CTRL_ERR];
+    if (w[CTRL_INFO] != 0 && info == 0) info = w[CTRL_INFO];
   }
   if (info != 0 || err != 0) {
-    GBTA_CUDA(cudaMemsetAsync(s->d_ctrl, 0, CTRL_INTS * sizeof(int), s->stream));
-    GBTA_CUDA(cudaMemsetAsync(s->d_ctrl2, 0, CTRL_INTS * sizeof(int), s->stream));
+    GBTA_CUDA(cudaMemsetAsync(s->d_ctrl, 0, 2 * CTRL_INTS * sizeof(int), s->stream));
     GBTA_CUDA(cudaStreamSynchronize(s->stream));
   }
   if (err == 1) return fail(GBTA_ERR_TIMEOUT, "a kernel wait exceeded the wait limit; the launch was abandoned");
