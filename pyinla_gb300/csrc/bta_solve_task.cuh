@@ -17,7 +17,7 @@
 // over the whole CTA) between the neighbour's publication and its own.  Solution tiles go
 // from task to task as words that carry their own readiness (st_word, wait_word): the chain
 // is bound by a store and a load across the chip and ~11 FP64 instructions of 64 cycles, a
-// tile's hop takes 1.40 us at b = 333 and 1.65 at b = 768 (2.3 with a store, a released
+// tile's hop takes 1.35 us at b = 333 and 1.57 at b = 768 (2.3 with a store, a released
 // flag, its poll and a reload, and the additions of absent columns).  The forward sweep also leaves the arrow contribution R_i(:,r) y(i,r) of each tile in a partial
 // buffer, after publishing the tile and under a flag of its own (off the chain), and
 // the arrow task sums the partials in a fixed order.
@@ -82,13 +82,27 @@ static __device__ __forceinline__ void cta_gemv(const double* Ms, const double* 
   }
 }
 
-// V <- the solution words of tile gi (rows valid), as they are written; a barrier.  False,
-// uniformly, when a wait was given up.
-static __device__ __forceinline__ bool vec_wait(double* V, const SolveArgs& p, int dir, int gi, int rows) {
+// V <- the solution words of tile gi (rows valid), as they are written; a barrier.  `lazy`:
+// a tile not there yet is watched by one thread with sleeps in between (the newest tile of the
+// chain is awaited by up to two block rows of tasks at once, and all of them polling every word
+// of it slowed the hop that the chain waits for: 1.66 -> 1.57 us at b = 768, 1.50 -> 1.40 at b =
+// 333 with two chains).  False, uniformly, when a wait was given up.
+constexpr int LAZY_DEPS = 6;   // dependencies after which a task is not close to its turn
+static __device__ __forceinline__ bool vec_wait(double* V, const SolveArgs& p, int dir, int gi, int rows,
+                                                bool lazy = false) {
   const int row = threadIdx.x / NC, col = threadIdx.x % NC;
-  double v = 0.0;
+  const bool mine = row < rows && col < p.nc;
+  const double* w = mine ? sol_words(p, dir, col, gi) + row : nullptr;
+  long long x = mine ? ld_word(w) : 0ll;
+  if (lazy && !__syncthreads_and(x != WORD_EMPTY)) {
+    if (threadIdx.x == 0 && x == WORD_EMPTY) {
+      for (int k = 0; k < 64 && (x = ld_word(w)) == WORD_EMPTY; ++k) __nanosleep(300);
+    }
+    __syncthreads();
+  }
+  double v = __longlong_as_double(x);
   bool ok = true;
-  if (row < rows && col < p.nc) ok = wait_word(p.c, sol_words(p, dir, col, gi) + row, v);
+  if (x == WORD_EMPTY) ok = wait_word(p.c, w, v);
   V[row * NC + col] = v;
   return __syncthreads_and(ok);
 }
@@ -364,7 +378,7 @@ static __device__ __forceinline__ bool solve_task(const SolveArgs& p, int t, uns
       }
       tile_load(Ts, d.t);   // the matrix tile does not depend on other tasks
       if (d.vtile >= 0) {
-        if (!(ok = vec_wait(Vs, p, dir, d.vtile, d.vrows))) break;
+        if (!(ok = vec_wait(Vs, p, dir, d.vtile, d.vrows, ndep - st > LAZY_DEPS))) break;
       } else {
         if (!(ok = cta_wait(c, c.flags + fo + ntile, nullptr, &s_ok))) break;
         vec_load(Vs, p, arrow_row0, d.vrows);
