@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_batch(const FactorArgs* __rest
   }
 }
 
-__global__ void __launch_bounds__(NT, 1) k_selinv_batch(const SelinvArgs* __restrict__ inst,
+__global__ void __launch_bounds__(NT, OZS_CTAS_PER_SM) k_selinv_batch(const SelinvArgs* __restrict__ inst,
                                                         const int2* __restrict__ order, int ntotal, Ctl c) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int s_ok, s_t, s_ready;
