@@ -136,11 +136,11 @@ int gbta_get_twist(const gbta_solver* s);
  * of both streams are read by gbta_status. */
 int gbta_set_selinv_overlap(gbta_solver* s, int enable);
 
-/* Persistent CTAs per SM of the dataflow launches (0, the default: as many as the
- * kernel's registers and shared memory allow for the factorization and the selected
- * inversion, one for the sweeps, whose latency-bound chain runs fastest so;
- * GBTA_CTAS_PER_SM in the environment sets the initial value).  No reference
- * counterpart (a launch-shape setting). */
+/* Persistent CTAs per SM of the dataflow launches (0, the default: for the
+ * factorization and the selected inversion as many as the kernel's registers and shared
+ * memory allow, fewer where the blocks are so narrow that the chain of block columns is
+ * the limit; for the sweeps one, two for wide blocks; GBTA_CTAS_PER_SM in the environment
+ * sets the initial value).  No reference counterpart (a launch-shape setting). */
 int gbta_set_ctas_per_sm(gbta_solver* s, int n);
 
 /* Task tracing (off by default).  When enabled, every dataflow kernel launched by

@@ -230,6 +230,29 @@ gbta::LaunchCtl next_launch(gbta_solver* s, int ntasks) {
   return lc;
 }
 
+// CTAs per SM of the tensor-core factorization and selected inversion, unless set
+// otherwise (0: all that fit).  Where the column chain is the limit, more CTAs only take
+// issue slots and polls from the tasks on the chain; one per SM is faster until a link's
+// other tiles, about chains * B^2 / 2 of them with the whole pattern in use, keep the SMs
+// busy longer than the chain takes to come round.  Random dense blocks on 152 SMs, two
+// chains (one chain crosses at B sqrt(2) times as wide, as the product says):
+//   factorization   one against two CTAs: b = 128 0.558 and 0.591 ms, b = 333 5.27 and 5.47,
+//                   b = 400 6.32 and 6.54, b = 480 7.76 and 7.63 (one chain: b = 544 10.02 and
+//                   10.43, b = 768 15.41 and 14.92);
+//   inversion       one, two, three CTAs: b = 256 3.01, 3.11, 3.16 ms, b = 333 4.42, 4.43,
+//                   4.53, b = 400 6.10, 5.31, 5.48, b = 480 8.19, 6.25, 6.44, b = 544 10.87,
+//                   7.82, 7.52 (one chain: b = 333 5.21, 5.36, 5.44, b = 544 8.74, 8.52, 8.74).
+// Banded couplings would cross later (half the tiles are left out), but that is known on the
+// device only.
+int factor_ctas(const gbta_solver* s) {
+  const long long tiles = (s->g.twisted() ? 2ll : 1ll) * s->g.B * s->g.B;
+  return 4 * tiles <= 9ll * s->nsm ? 1 : 0;
+}
+int selinv_ctas(const gbta_solver* s) {
+  const long long tiles = (s->g.twisted() ? 2ll : 1ll) * s->g.B * s->g.B;
+  return 5 * tiles <= 8ll * s->nsm ? 1 : tiles <= 3ll * s->nsm ? 2 : 0;
+}
+
 // The same for a launch on the side stream (overlapped inversion).
 gbta::LaunchCtl next_side_launch(gbta_solver* s, int ntasks) {
   const int e0 = s->epoch;
@@ -590,7 +613,8 @@ static int factor_async(gbta_solver* s, double* D, double* L, double* R, double*
     gbta::launch_coupling_kfirst(s->g, L, s->d_kf, s->stream);
   }
   gbta::launch_clear_feeders(s->g, s->d_flags, s->d_wpub, s->stream);
-  const gbta::LaunchCtl lc = next_launch(s, s->n_ftasks);
+  gbta::LaunchCtl lc = next_launch(s, s->n_ftasks);
+  if (s->ctas_per_sm == 0 && s->method == GBTA_METHOD_OZAKI) lc.ctas_per_sm = factor_ctas(s);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[0], s->stream));
   s->fac_digits = s->method == GBTA_METHOD_OZAKI;
   if (s->method == GBTA_METHOD_OZAKI)
@@ -772,8 +796,9 @@ static int selinv_async(gbta_solver* s, double* D, double* L, double* R, double*
   s->fac_evt = false;
   if (int r = over ? reset_side_ticket(s) : reset_ticket(s)) return r;
   gbta::LaunchCtl lc = over ? next_side_launch(s, s->n_stasks) : next_launch(s, s->n_stasks);
-  // (its grid is the full one: the CTAs that find no slot next to the sweeps' CTAs,
-  // which were launched first and keep one per SM, start when those exit)
+  // (overlapped, the CTAs that find no slot next to the sweeps' CTAs, which were launched
+  // first and keep one per SM, start when those exit)
+  if (s->ctas_per_sm == 0 && ozaki) lc.ctas_per_sm = selinv_ctas(s);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[2], st));
   if (ozaki)   // (its pre-pass reads the G tiles: from the workspace when overlapped)
     gbta::launch_selinv_oz(g, over ? SD : D, over ? SL : L, over ? SR : R, T, SD, SL, SR, ST, use_arrow,

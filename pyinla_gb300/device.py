@@ -69,7 +69,7 @@ class BtaHandle:
         _lib.check(self.lib.gbta_set_method(self.ptr, int(method)))
 
     def set_ctas_per_sm(self, n: int) -> None:
-        """Persistent CTAs per SM of the dataflow launches (0: as many as fit)."""
+        """Persistent CTAs per SM of the dataflow launches (0: chosen by block width)."""
         _lib.check(self.lib.gbta_set_ctas_per_sm(self.ptr, int(n)))
 
     def set_selinv_overlap(self, enable: bool) -> None:
