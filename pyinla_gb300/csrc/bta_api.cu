@@ -242,21 +242,36 @@ gbta::LaunchCtl next_launch(gbta_solver* s, int ntasks) {
 // busy longer than the chain takes to come round.  Random dense blocks on 152 SMs, two
 // chains (one chain crosses at B sqrt(2) times as wide, as the product says):
 //   factorization   one against two CTAs: b = 128 0.558 and 0.591 ms, b = 333 5.27 and 5.47,
-//                   b = 400 6.32 and 6.54, b = 480 7.76 and 7.63 (one chain: b = 544 10.02 and
-//                   10.43, b = 768 15.41 and 14.92);
+//                   b = 448 6.99 and 7.07, b = 480 7.76 and 7.63 (one chain: b = 608 11.23 and
+//                   11.66, b = 768 15.41 and 14.92);
 //   inversion       one, two, three CTAs: b = 256 3.01, 3.11, 3.16 ms, b = 333 4.42, 4.43,
 //                   4.53, b = 400 6.10, 5.31, 5.48, b = 480 8.19, 6.25, 6.44, b = 544 10.87,
 //                   7.82, 7.52 (one chain: b = 333 5.21, 5.36, 5.44, b = 544 8.74, 8.52, 8.74).
-// Banded couplings would cross later (half the tiles are left out), but that is known on the
-// device only.
-int factor_ctas(const gbta_solver* s) {
-  const long long tiles = (s->g.twisted() ? 2ll : 1ll) * s->g.B * s->g.B;
-  return 4 * tiles <= 9ll * s->nsm ? 1 : 0;
+// Of banded couplings the structurally zero tiles are left out, and the lines lie where the
+// live ones are as many.  Only the device knows how many those are, so between the dense line
+// and three times its tiles the grid is a full one and its CTAs decide (cta_spare).  SPDE
+// models, ~0.6 of the tiles live: factorization at b = 484 one CTA 3.98, two 4.09 ms, b = 576
+// 4.52 and 4.66, b = 625 5.23 and 5.19; inversion one, two, three CTAs b = 400 2.65, 2.75,
+// 2.79, b = 576 4.67, 3.83, 3.94, b = 676 7.34, 5.00, 4.99.
+// num1 / den1, num2 / den2: live tiles per SM up to which one CTA and two stay.
+void ctas_by_width(const gbta_solver* s, gbta::LaunchCtl& lc, int num1, int den1, int num2, int den2) {
+  const gbta::Geom& g = s->g;
+  const long long chains = g.twisted() ? 2 : 1, tiles = chains * g.B * g.B, nsm = s->nsm;
+  if (den1 * tiles <= num1 * nsm) {
+    lc.ctas_per_sm = 1;
+    return;
+  }
+  if (den2 * tiles <= num2 * nsm) lc.ctas_per_sm = 2;
+  if (g.nt < 2 || den2 * tiles > 3 * num2 * nsm) return;
+  lc.spare.kf = s->d_kf;
+  lc.spare.rows = (g.nt - 1) * g.B;
+  lc.spare.B = g.B;
+  lc.spare.nsm = s->nsm;
+  lc.spare.lim1 = num1 * nsm * (g.nt - 1) / (den1 * chains);
+  lc.spare.lim2 = num2 * nsm * (g.nt - 1) / (den2 * chains);
 }
-int selinv_ctas(const gbta_solver* s) {
-  const long long tiles = (s->g.twisted() ? 2ll : 1ll) * s->g.B * s->g.B;
-  return 5 * tiles <= 8ll * s->nsm ? 1 : tiles <= 3ll * s->nsm ? 2 : 0;
-}
+void factor_ctas(const gbta_solver* s, gbta::LaunchCtl& lc) { ctas_by_width(s, lc, 27, 10, 27, 10); }
+void selinv_ctas(const gbta_solver* s, gbta::LaunchCtl& lc) { ctas_by_width(s, lc, 5, 3, 3, 1); }
 
 // The same for a launch on the side stream (overlapped inversion).
 gbta::LaunchCtl next_side_launch(gbta_solver* s, int ntasks) {
@@ -619,7 +634,7 @@ static int factor_async(gbta_solver* s, double* D, double* L, double* R, double*
   }
   gbta::launch_clear_feeders(s->g, s->d_flags, s->d_wpub, s->stream);
   gbta::LaunchCtl lc = next_launch(s, s->n_ftasks);
-  if (s->ctas_per_sm == 0 && s->method == GBTA_METHOD_OZAKI) lc.ctas_per_sm = factor_ctas(s);
+  if (s->ctas_per_sm == 0 && s->method == GBTA_METHOD_OZAKI) factor_ctas(s, lc);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[0], s->stream));
   s->fac_digits = s->method == GBTA_METHOD_OZAKI;
   if (s->method == GBTA_METHOD_OZAKI)
@@ -803,7 +818,7 @@ static int selinv_async(gbta_solver* s, double* D, double* L, double* R, double*
   gbta::LaunchCtl lc = over ? next_side_launch(s, s->n_stasks) : next_launch(s, s->n_stasks);
   // (overlapped, the CTAs that find no slot next to the sweeps' CTAs, which were launched
   // first and keep one per SM, start when those exit)
-  if (s->ctas_per_sm == 0 && ozaki) lc.ctas_per_sm = selinv_ctas(s);
+  if (s->ctas_per_sm == 0 && ozaki) selinv_ctas(s, lc);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[2], st));
   if (ozaki)   // (its pre-pass reads the G tiles: from the workspace when overlapped)
     gbta::launch_selinv_oz(g, over ? SD : D, over ? SL : L, over ? SR : R, T, SD, SL, SR, ST, use_arrow,

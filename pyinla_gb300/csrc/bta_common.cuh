@@ -324,6 +324,22 @@ __device__ __forceinline__ int cta_ticket(const Ctl& c, int* s_t) {
   return *s_t;
 }
 
+// Whether this CTA leaves at once (see SpareRule; uniform).  The first nsm CTAs of a grid,
+// and the second, are placed one per SM, so those that stay are spread evenly; the tickets go
+// to whoever is there.  s: a shared word.
+__device__ __forceinline__ bool cta_spare(const SpareRule& r, int* s) {
+  if (!r.kf || (int)blockIdx.x < r.nsm) return false;
+  if (threadIdx.x == 0) *s = 0;
+  __syncthreads();
+  int live = 0;
+  for (int k = threadIdx.x; k < r.rows; k += NT) live += r.B - r.kf[k];
+  atomicAdd(s, live);
+  __syncthreads();
+  const long long n = *s;
+  __syncthreads();
+  return (int)blockIdx.x >= (n <= r.lim1 ? 1 : n <= r.lim2 ? 2 : 8) * r.nsm;
+}
+
 // A tile view into a row-major matrix: rows x cols valid elements (<= TS each).
 struct Tile {
   const double* p;

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_oz(FactorArgs p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
+  if (cta_spare(p.spare, &s_t)) return;
   oz_pipe_init(&pipe, p.c);
   const OzFactorSmem sm = oz_factor_smem(smem_raw, &s_ok, &s_ready, &pipe);
   while (true) {
@@ -73,6 +74,7 @@ void launch_factor_oz(const Geom& g, double* D, double* L, double* R, double* T,
   p.diag_pre = diag_pre;
   p.kf = kf;
   p.wpub = wpub;
+  p.spare = lc.spare;
   p.c.ctrl = lc.ctrl;
   p.c.flags = lc.flags;
   p.c.epoch = lc.epoch;

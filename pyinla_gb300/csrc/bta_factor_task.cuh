@@ -52,6 +52,7 @@ struct FactorArgs {
                         // (smem_potrf's Wg; WORD_EMPTY at launch), or null without FT_FEEDQ
   const int* kf;        // [(nt-1)*B] first column tile of each coupling-slot row tile that
                         // can be nonzero (launch_coupling_kfirst), or null
+  SpareRule spare;
   Ctl c;
 };
 

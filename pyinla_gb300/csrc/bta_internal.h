@@ -128,6 +128,17 @@ struct Geom {
 // are three or more blocks (two chains of about nt/2 blocks), else the plain order.
 inline int default_sep(int nt) { return nt >= 3 ? nt / 2 : nt - 1; }
 
+// CTAs of a full grid that are not wanted where the couplings turn out to be banded: with at
+// most lim1 live coupling tiles (Σ (B - kf) over the slots' row tiles) one CTA per SM stays,
+// with at most lim2 two.  kf null: all stay.
+struct SpareRule {
+  const int* kf = nullptr;
+  int rows = 0;
+  int B = 0;
+  int nsm = 0;
+  long long lim1 = 0, lim2 = 0;
+};
+
 struct LaunchCtl {
   int* ctrl;
   int* flags;
@@ -139,6 +150,7 @@ struct LaunchCtl {
   int nsm = 0;                  // > 0: size the grid from the kernel's occupancy (launch_grid)
   int ctas_per_sm = 0;          // CTAs per SM (0: as many as fit)
   int ntasks = 0;               // never more CTAs than tasks
+  SpareRule spare;
 };
 
 // Persistent grid of a kernel with `threads` threads and `smem` bytes of dynamic

@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(NT, OZS_CTAS_PER_SM) k_selinv_oz(SelinvArgs p)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_ok, s_t, s_ready;
   __shared__ OzPipe pipe;
+  if (cta_spare(p.spare, &s_t)) return;
   oz_pipe_init(&pipe, p.c);
   while (true) {
     const int t = cta_ticket(p.c, &s_t);
@@ -182,6 +183,7 @@ void launch_selinv_oz(const Geom& g, const double* D, const double* L, const dou
   p.part = part;
   p.part_flag = part_flag;
   p.merged = 1;
+  p.spare = lc.spare;
   p.c.ctrl = lc.ctrl;
   p.c.flags = lc.flags;
   p.c.epoch = lc.epoch;

@@ -67,6 +67,7 @@ struct SelinvArgs {
   double* part;         // Ozaki, merged task list: [nt*B][TS*TS] partial sums of the
   int* part_flag;       // sub-diagonal tiles and their epoch-stamped flags [nt*B]
   int merged;           // the task list is selinv_task_list(g, true)
+  SpareRule spare;
   Ctl c;
 };
 

@@ -1,6 +1,7 @@
 """Narrow blocks: the factorization and the selected inversion run fewer CTAs per SM below a
-block width (two chains: 13 tiles for the factorization, 11 and 15 for the inversion on 152
-SMs; one chain: 18, 15 and 21).
+block width (two chains: 14 tiles for the factorization, 11 and 15 for the inversion on 152
+SMs; one chain: 20, 15 and 21), later with banded couplings, whose live tiles the kernels
+count themselves.
 
 The results do not depend on the number of CTAs (every sum has a fixed order), so on both
 sides of each line the default is equal, bit for bit, to a launch pinned to two per SM; both
@@ -13,8 +14,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("twist", [True, False])
-@pytest.mark.parametrize("b", [20, 352, 353, 416, 417, 480, 481, 577, 673])
-def test_any_number_of_ctas(b, twist):
+@pytest.mark.parametrize("b,banded", [(b, False) for b in (20, 352, 353, 448, 449, 480, 481, 640, 673)] +
+                         [(b, True) for b in (448, 481, 576, 609, 640, 704)])
+def test_any_number_of_ctas(b, banded, twist):
     import torch
 
     from oracle import bta_oracle as oracle
@@ -22,6 +24,9 @@ def test_any_number_of_ctas(b, twist):
     from pyinla_gb300.synthetic import random_bta
     nt, a = 4, 3
     Q = random_bta(nt, b, a, seed=b)
+    if banded:
+        Q = [q.clone() for q in Q]
+        Q[1].copy_(torch.tril(torch.triu(Q[1], -20), 20))
     h = BtaHandle.get(b, nt, a, True)
     h.set_stream(current_stream_ptr())
     h.set_selinv_overlap(False)
