@@ -387,7 +387,10 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
   CREATE_CUDA(cudaMemsetAsync(s->d_faux, 0, ntile * sizeof(int), s->stream));
   CREATE_CUDA(cudaMalloc(&s->d_dpre, 2 * ntile * sizeof(int)));
   CREATE_CUDA(cudaMemsetAsync(s->d_dpre, 0, 2 * ntile * sizeof(int), s->stream));
-  if (nt > 1) CREATE_CUDA(cudaMalloc(&s->d_kf, (size_t)(nt - 1) * s->g.B * sizeof(int)));
+  if (nt > 1) {   // (every tile live until a factorization has looked)
+    CREATE_CUDA(cudaMalloc(&s->d_kf, (size_t)(nt - 1) * s->g.B * sizeof(int)));
+    CREATE_CUDA(cudaMemsetAsync(s->d_kf, 0, (size_t)(nt - 1) * s->g.B * sizeof(int), s->stream));
+  }
   CREATE_CUDA(cudaMalloc(&s->d_ld, (nt + 2) * sizeof(double)));
   CREATE_CUDA(cudaMallocHost(&s->h_ctrl, 2 * CTRL_INTS * sizeof(int)));
   CREATE_CUDA(cudaMemsetAsync(s->d_ctrl, 0, 2 * CTRL_INTS * sizeof(int), s->stream));
