@@ -627,9 +627,10 @@ __device__ __forceinline__ double rcp3_fma(double d) {
 // fp32 reciprocal of the leading 24 significand bits; rcp_finish takes d's significand m
 // (2^52 <= m < 2^53) and the seed Y0 (24 bits, Y0 2^-24 ~ 2^52 / m), forms delta = m Y0 -
 // 2^76 modulo 2^64 (|delta| < 2^54) and Y = Y0 2^29 (1 - delta 2^-76 + (delta 2^-76)^2),
-// the reciprocal's significand.  A positive d outside the range where d and 1/d are normal
-// numbers gives what rcp3_fma's flushing seed leads to: 0 where 1/d is subnormal, NaN for a
-// zero, subnormal or infinite d; so does a negative d or a NaN (a failed pivot anyway).
+// the reciprocal's significand.  Where 1/d is subnormal (d from 2^1022 on) it is Y shifted by
+// one or two places, truncated (50 bits at least).
+// A zero, subnormal or infinite d gives NaN; so does a negative d or a NaN (a failed pivot
+// anyway).
 __device__ __forceinline__ float rcp_seed(double d) {
   const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
   const float f = __uint_as_float(0x3f800000u | (__funnelshift_l(lo, hi, 3) & 0x7fffffu));
@@ -647,11 +648,11 @@ __device__ __forceinline__ double rcp_finish(double d, float seed) {
   const unsigned sq = (unsigned)(((long long)dh * dh) >> 20);
   const long long q2 = (long long)(((unsigned long long)sq * Y0) >> 24);
   const long long Y = ((long long)Y0 << 29) - ((c - q2 + (1ll << 14)) >> 15);
-  const unsigned eb = (2044u << 20) - (hi & 0x7ff00000u);
-  const long long bits = (long long)((unsigned long long)eb << 32) + Y;
-  const unsigned ex = hi >> 20;
-  const int odd = ex - 2045u < 2u ? 0 : 0x7ff80000;   // (high words of 0 and NaN)
-  return ex - 1u < 2044u ? __longlong_as_double(bits) : __hiloint2double(odd, 0);
+  // (the exponent word and the shift depend on d alone: one shift and one addition behind Y)
+  const unsigned ex = hi >> 20, sub = ex - 2044u;   // sub: 1 or 2 where 1/d is subnormal
+  const unsigned eb = ex - 1u < 2044u ? (2044u << 20) - (hi & 0x7ff00000u) : sub - 1u < 2u ? 0u : 0x7ffu << 20;
+  const unsigned n = ex - 1u < 2044u ? 0u : sub - 1u < 2u ? sub : 2u;   // (2: a NaN's quarter stays one)
+  return __longlong_as_double((long long)((unsigned long long)eb << 32) + (Y >> n));
 }
 
 // Register slots of the update warps of smem_potrf.  Slot s < 14 holds column s + 2
