@@ -767,7 +767,9 @@ __device__ __forceinline__ void potrf_update_warp(double* S, const double* Wt, i
 // the pivot that look-ahead column p+4 needs.
 // With Wg (TS x TS words of global memory holding WORD_EMPTY) every pivot k is also written
 // there as it forms, row k: w_{:,k} with d_k in w_kk's place, for tasks on other SMs that
-// follow the elimination (wait_word).
+// follow the elimination (wait_word).  A non-positive pivot and those after it are not: the
+// followers wait until the launch is given up, so no later tile starts from this one, and no
+// row behind it can be reported in its place.
 // Out of line: its code is ~25 KB, once per kernel is enough.
 static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_addr, double* Wg) {
   double* S = reinterpret_cast<double*>(__cvta_shared_to_generic(s_addr));
@@ -779,6 +781,7 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
     double a = S[r * LDS];         // column k through pivot k-1 (column 0 of U is column 0 of S)
     double an = S[r * LDS + 1];    // column k+1 through pivot k-1 (column 1: no update yet)
     double dk = 1.0;               // lane k keeps d_k
+    int bad = 0;                   // the first non-positive pivot
 #pragma unroll 1
     for (int k = 0; k < TS; ++k) {
       const double d = __shfl_sync(0xffffffffu, a, k);
@@ -798,10 +801,10 @@ static __device__ __noinline__ int smem_potrf_at(unsigned s_addr, unsigned w_add
         Wt[k * TS + r] = w;
         nbar_arrive(POTRF_BAR_L + (k & 7));
       }
-      if (Wg) st_word(Wg + k * TS + r, r == k ? d : w);
+      if (!bad && !positive_bits(d)) bad = k + 1;   // (uniform)
+      if (Wg && !bad) st_word(Wg + k * TS + r, r == k ? d : w);
     }
-    const unsigned bad = __ballot_sync(0xffffffffu, !positive_bits(dk));
-    if (r == 0) s_info = bad ? __ffs(bad) : 0;
+    if (r == 0) s_info = bad;
     // L = U D^{-1/2}: the last two columns here, the others by warps 1-3, which have them
     // complete two pivots earlier
     const double y = rsqrt3(dk);
