@@ -46,6 +46,7 @@ struct gbta_solver {
   int ctas_per_sm = 0;   // persistent CTAs per SM (0: as many as fit)
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
+  cudaStream_t queued_on = nullptr;   // stream of the last launch (compared only)
   unsigned long long wait_ns = 20ull * 1000 * 1000 * 1000;
   int epoch = 0;
 
@@ -228,6 +229,7 @@ gbta::LaunchCtl next_launch(gbta_solver* s, int ntasks) {
   lc.ctas_per_sm = s->ctas_per_sm;
   lc.ntasks = ntasks;
   lc.stream = s->stream;
+  s->queued_on = s->stream;
   if (s->d_trace && ntasks <= s->trace_cap) {
     lc.trace = s->d_trace;
     s->trace_n = ntasks;
@@ -361,7 +363,7 @@ int gbta_create(int b, int nt, int a, gbta_solver** out) {
     if (ms > 0.0) s->wait_ns = (unsigned long long)(ms * 1e6);
   }
   CREATE_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
-  s->stream = s->own_stream;
+  s->stream = s->queued_on = s->own_stream;
   CREATE_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
   CREATE_CUDA(cudaEventCreateWithFlags(&s->ev_fac, cudaEventDisableTiming));
   CREATE_CUDA(cudaEventCreateWithFlags(&s->ev_sel, cudaEventDisableTiming));
@@ -587,10 +589,17 @@ size_t gbta_workspace_bytes(const gbta_solver* s) {
 int gbta_status(gbta_solver* s) {
   if (int r = check_solver(s)) return r;
   // the sticky words of both control blocks (the side stream's: an overlapped inversion), by one
-  // copy behind the stream's work (two blocking copies after it took 22 us a call, this 12)
+  // copy behind the stream's work (two blocking copies after it took 22 us a call, this 12).
+  // When the stream was changed since the last launch, by a blocking copy: it also comes after
+  // what was queued on the default stream, and the new stream's need not.
   GBTA_CUDA(cudaStreamSynchronize(s->side));
-  GBTA_CUDA(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, 2 * CTRL_INTS * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  GBTA_CUDA(cudaStreamSynchronize(s->stream));
+  if (s->queued_on == s->stream) {
+    GBTA_CUDA(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, 2 * CTRL_INTS * sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    GBTA_CUDA(cudaStreamSynchronize(s->stream));
+  } else {
+    GBTA_CUDA(cudaStreamSynchronize(s->stream));
+    GBTA_CUDA(cudaMemcpy(s->h_ctrl, s->d_ctrl, 2 * CTRL_INTS * sizeof(int), cudaMemcpyDeviceToHost));
+  }
   GBTA_CUDA(cudaGetLastError());
   int info = 0, err = 0;
   for (const int* w : {s->h_ctrl, s->h_ctrl + CTRL_INTS}) {
