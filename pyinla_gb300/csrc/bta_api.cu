@@ -682,6 +682,35 @@ int gbta_pobtf(gbta_solver* s, double* D, double* L) {
 }
 
 // ---------------------------------------------------------------- solves
+// CTAs per SM of a launch of nc columns (trans: 0 forward, 1 backward, 2 both sweeps), unless
+// set otherwise.  The sweeps run one: their chain needs few, and more spend the SMs' issue slots
+// and memory traffic on waiting tasks (both sweeps at nt = 128, b = 1024: 7.0 ms against 7.9
+// with two and 8.7 with three).  Two where a task's other products (two block rows of tiles)
+// take longer than the chain needs to come round to the next of the SMs it is shared out to.
+// One column: from 40 tiles per block edge with two chains (b = 1280: 2.49 ms against 2.59, b =
+// 2048: 2.32 against 2.97, b = 3072: 3.08 against 4.59; b = 1024: 2.58 against 2.31), twice that
+// with one (b = 2560: 3.61 ms either way); next to an overlapped inversion one and two leave the
+// same two of its CTAs' places on each SM.
+// With two to four columns the FP64 instructions of a tile's products double and more, and a
+// second CTA's take the pipe from the chain's link, so the lines lie higher.  Four columns, one
+// CTA and two, ms:
+//   one chain    b = 2600 1.15, 1.41; b = 3500 1.89, 1.89; b = 4200 2.45, 2.26 (both sweeps);
+//   backward     b = 1500, nt = 8 0.86, 1.03; b = 2048, nt = 3, 8, 12 0.57, 0.56; 1.37, 1.40;
+//                2.00, 1.95; b = 2304, nt = 6 1.36, 1.26;
+//   both sweeps  b = 1280, nt = 12 2.05, 2.60; b = 2048, nt = 8, 12 2.92, 3.04; 4.12, 4.13; b =
+//                2304, nt = 3, 6, 12 1.50, 1.53; 2.76, 2.79; 5.23, 4.65; b = 2600, nt = 3 1.79, 1.76;
+//   forward      ends on the separator alone, whose tiles have the products of two neighbours,
+//                one block of nt: b = 2048, nt = 12 2.16, 2.21; b = 2304, nt = 6, 12 1.44, 1.55;
+//                2.71, 2.49; b = 2816, nt = 6 1.90, 1.95; b = 3072, nt = 3, 8 1.17, 1.24; 2.85, 2.61.
+// With two columns two CTAs are worth up to 10 % more there than with four.
+static int sweep_ctas(const gbta::Geom& g, int nc, int trans) {
+  const long long tiles = (g.twisted() ? 2 : 1) * g.B;
+  if (nc == 1) return tiles >= 80 ? 2 : 1;
+  if (!g.twisted()) return tiles >= 110 ? 2 : 1;
+  if (trans == 0) return tiles * (g.nt - 1) >= 125ll * g.nt ? 2 : 1;
+  return tiles >= (trans == 1 ? 128 : 140) ? 2 : 1;
+}
+
 static int solve_async(gbta_solver* s, const double* D, const double* L, const double* R, const double* T, double* B,
                        int nrhs, int trans, int use_arrow) {
   if (int r = check_solver(s)) return r;
@@ -692,22 +721,13 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
   // both sweeps in one launch where the flag array has room for the second sweep's flags
   // (every geometry but b <= 32), else one after the other
   const bool both = trans == 2 && gbta::solve_both_fits(s->g);
-  const int sweep_ctas = s->g.B * (s->g.twisted() ? 2 : 1) >= 80 ? 2 : 1;   // (see below)
   const int ntasks = (s->g.nt * s->g.B + (use_arrow ? 1 : 0)) * (both ? 2 : 1);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[4], s->stream));
   for (int c0 = 0; c0 < nrhs; c0 += gbta::SOLVE_NC) {
     const int nc = nrhs - c0 < gbta::SOLVE_NC ? nrhs - c0 : gbta::SOLVE_NC;
     if (int r = reset_ticket(s)) return r;
     gbta::LaunchCtl lc = next_launch(s, ntasks);
-    // The sweeps run one CTA per SM unless set otherwise: their chain needs few, and more
-    // spend the SMs' issue slots and memory traffic on waiting tasks (both sweeps at nt = 128,
-    // b = 1024: 7.0 ms against 7.9 with two and 8.7 with three).  Two where a task's other
-    // products (two block rows of tiles) take longer than the chain needs to come round to the
-    // next of the SMs it is shared out to: from 40 tiles per block edge with two chains (b =
-    // 1280: 2.49 ms against 2.59, b = 2048: 2.32 against 2.97, b = 3072: 3.08 against 4.59; b =
-    // 1024: 2.58 against 2.31), twice that with one (b = 2560: 3.61 ms either way).  Next to
-    // an overlapped inversion they leave the same two of its CTAs' places on each SM.
-    if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas;
+    if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas(s->g, nc, trans);
     if (both) {
       gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, 0, use_arrow, s->d_arrow_part, s->d_wpub, lc, 1);
     } else {
@@ -715,7 +735,7 @@ static int solve_async(gbta_solver* s, const double* D, const double* L, const d
         if (tr == 1 && trans == 2) {   // the second sweep of trans = 2: its own launch
           if (int r = reset_ticket(s)) return r;
           lc = next_launch(s, ntasks);
-          if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas;
+          if (s->ctas_per_sm == 0) lc.ctas_per_sm = sweep_ctas(s->g, nc, trans);
         }
         gbta::launch_solve(s->g, D, L, R, T, B + c0, nrhs, nc, tr, use_arrow, s->d_arrow_part,
                            s->d_wpub, lc);
@@ -829,7 +849,7 @@ static int selinv_async(gbta_solver* s, double* D, double* L, double* R, double*
   if (int r = over ? reset_side_ticket(s) : reset_ticket(s)) return r;
   gbta::LaunchCtl lc = over ? next_side_launch(s, s->n_stasks) : next_launch(s, s->n_stasks);
   // (overlapped, the CTAs that find no slot next to the sweeps' CTAs, which were launched
-  // first and keep one per SM, start when those exit)
+  // first and keep one or two per SM, start when those exit)
   if (s->ctas_per_sm == 0 && ozaki) selinv_ctas(s, lc);
   if (s->timing) GBTA_CUDA(cudaEventRecord(s->tev[2], st));
   if (ozaki)   // (its pre-pass reads the G tiles: from the workspace when overlapped)
