@@ -723,11 +723,16 @@ static __device__ __forceinline__ bool selinv_oz_task(const SelinvArgs& p, int t
     trace_clear_marks(c, t);
     trace_put(c, t, 3, np);   // product steps (a diagonal task overwrites it below)
     unsigned long long* red = reinterpret_cast<unsigned long long*>(red4);
-    double sv[2][4];   // this thread's elements of X
+    // this thread's elements of X; of a diagonal tile the lower triangle only: the other
+    // elements are overwritten by their mirror images below, with no barrier in between
+    double sv[2][4];
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) sv[n][q] = X[oz_row(n, q) * LDS + oz_col(n, q)];
+      for (int q = 0; q < 4; ++q) {
+        const int r = oz_row(n, q), cc = oz_col(n, q);
+        sv[n][q] = type != ST_DIAG || r >= cc ? X[r * LDS + cc] : 0.0;
+      }
     auto acc_to_x = [&](double* Y, const double (&v)[2][4]) {
 #pragma unroll
       for (int n = 0; n < 2; ++n)
