@@ -564,21 +564,19 @@ __device__ __forceinline__ void tile_diag_recip(const double* F, double* rd) {
 }
 
 // ---- register-resident tile factorization and triangular solves ------------------
-// In the triangular solves, thread (lane r, warp g) holds row r of the tile at the
-// eight columns c = g + 4q (q = 0..7) in registers, so every FP64 instruction has 32
-// useful lanes.  Columns are processed in order; the warp owning the current column
+// In the solve of a whole tile (smem_trsm_rlt), thread (lane r, warp g) holds row r of the
+// tile at the eight columns c = g + 4q (q = 0..7) in registers, so every FP64 instruction
+// has 32 useful lanes.  Columns are processed in order; the warp owning the current column
 // finalises it and publishes it through shared memory with one CTA barrier per column,
-// and every warp then updates its later columns with one FMA per element (the
-// Cholesky, smem_potrf below, splits the work differently).  The loops over
+// and every warp then updates its later columns with one FMA per element.  (The Cholesky,
+// smem_potrf, and the other solves, which give a row's columns to lanes of one warp and
+// need no barrier, split the work differently; see there.)  The loops over
 // columns and register slots are fully unrolled: the conditions "column c = g + 4q
 // is after column j" are written as a compile-time part plus a runtime part that
 // only the one boundary slot needs, because an FP64 instruction issued under a false
 // predicate still costs a full pipe slot.
 __device__ __forceinline__ bool col_after(int q, int j, int g) {   // g + 4q > j
   return 4 * q > j || (4 * q + 3 > j && g > j - 4 * q);
-}
-__device__ __forceinline__ bool col_before(int q, int j, int g) {  // g + 4q < j
-  return 4 * q + 3 < j || (4 * q < j && g < j - 4 * q);
 }
 
 // Named CTA barriers (ids 1 .. 15; id 0 is __syncthreads) for a producer warp that
@@ -612,18 +610,9 @@ __device__ __forceinline__ bool positive_bits(double x) {
   return b > 0 && b <= 0x7ff0000000000000ll;
 }
 
-// 1/d with the third-order refinement in three dependent FMAs (for a chain that counts
-// FP64 instructions): e = 1 - d y, y <- y + y (e + e^2).
-__device__ __forceinline__ double rcp3_fma(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
 // 1/d on the integer pipe, for a chain that waits on every reciprocal: an FP64 instruction
-// takes 64 cycles, so rcp3_fma costs 227 cycles (measured, dependent), this 120 with the
-// same error (at most 1.11e-16 relative over 2^20 values).  rcp_seed starts the hardware's
+// takes 64 cycles, so the hardware's seed with a third-order refinement in three dependent
+// FMAs costs 227 cycles (measured), this 120 with the same error (at most 1.11e-16 relative over 2^20 values).  rcp_seed starts the hardware's
 // fp32 reciprocal of the leading 24 significand bits; rcp_finish takes d's significand m
 // (2^52 <= m < 2^53) and the seed Y0 (24 bits, Y0 2^-24 ~ 2^52 / m), forms delta = m Y0 -
 // 2^76 modulo 2^64 (|delta| < 2^54) and Y = Y0 2^29 (1 - delta 2^-76 + (delta 2^-76)^2),
@@ -757,7 +746,8 @@ __device__ __forceinline__ void potrf_update_warp(double* S, const double* Wt, i
 // of the reciprocal, under its latency.  In the factorization kernel a tile takes 14.2k
 // cycles, ~405 a pivot (18k before the integer reciprocal, the update schedule and the
 // scaling of the first 30 columns beside the last two pivots): a column link at b = 128 or
-// 333 19.2 us instead of 20.3.
+// 333 took 19.2 us instead of 20.3 for it, and takes 15.4 with the solves that follow the
+// pivots (smem_trsm_follow).
 // Warps 1-3 apply every pivot to the later columns (potrf_update_warp), the column that
 // the pivot warp needs next first; each entry receives its updates in pivot order.
 // Barrier ids rotate over 8 (pivots) and 4 (look-ahead columns): before the pivot warp

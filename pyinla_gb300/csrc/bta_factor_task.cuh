@@ -647,7 +647,6 @@ static __device__ __forceinline__ bool factor_oz_task(const FactorArgs& p, int t
   int* erow_t = sm.erow_t;
   int* ecol_t = sm.ecol_t;
   int& s_ok = *sm.s_ok;
-  int& s_ready = *sm.s_ready;
   const Geom& g = p.g;
   const Ctl& c = p.c;
   int* info_slot = p.info ? p.info : c.ctrl + CTRL_INFO;

@@ -17,10 +17,12 @@
 // over the whole CTA) between the neighbour's publication and its own.  Solution tiles go
 // from task to task as words that carry their own readiness (st_word, wait_word): the chain
 // is bound by a store and a load across the chip and ~11 FP64 instructions of 64 cycles, a
-// tile's hop takes 1.35 us at b = 333 and 1.57 at b = 768 (2.3 with a store, a released
-// flag, its poll and a reload, and the additions of absent columns).  The forward sweep also leaves the arrow contribution R_i(:,r) y(i,r) of each tile in a partial
-// buffer, after publishing the tile and under a flag of its own (off the chain), and
-// the arrow task sums the partials in a fixed order.
+// tile's hop takes 1.35 us at b = 333 and 1.57 at b = 768 in a backward sweep of one chain and
+// one column (1.38 and 1.61 with two chains, up to 0.2 more in a forward one, 3.3 with four
+// columns; 2.3 with a store, a released flag, its poll and a reload, and the additions of
+// absent columns).  The forward sweep also leaves the arrow contribution R_i(:,r) y(i,r) of
+// each tile in a partial buffer, after publishing the tile and under a flag of its own (off the
+// chain), and the arrow task sums the partials in a fixed order.
 #pragma once
 
 #include "bta_common.cuh"
@@ -86,7 +88,7 @@ static __device__ __forceinline__ void cta_gemv(const double* Ms, const double* 
 // a tile not there yet is watched by one thread with sleeps in between (the newest tile of the
 // chain is awaited by up to two block rows of tasks at once, and all of them polling every word
 // of it slowed the hop that the chain waits for: 1.66 -> 1.57 us at b = 768, 1.50 -> 1.40 at b =
-// 333 with two chains).  False, uniformly, when a wait was given up.
+// 333 with two chains, when it was taken up).  False, uniformly, when a wait was given up.
 constexpr int LAZY_DEPS = 6;   // dependencies after which a task is not close to its turn
 static __device__ __forceinline__ bool vec_wait(double* V, const SolveArgs& p, int dir, int gi, int rows,
                                                 bool lazy = false) {
